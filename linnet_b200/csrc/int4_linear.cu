@@ -1,28 +1,49 @@
 // Row-count dispatch of the int4 linear layer, the counterpart of the generated
 // `_int4_linear` (src/backend/torch_source.cpp:1553-1570): few rows stream the
 // weight once through the decode kernel, many rows go to the tcgen05 dequant-GEMM.
-#include "common.cuh"
-
-namespace b200q {
-// Defined in int4_gemm_sm100.cu: whether the tcgen05 kernel takes this problem.
-bool int4_gemm_supports(int64_t rows, int64_t in, int64_t out, int64_t group, int32_t dtype,
-                        const void* x, const void* y);
-}  // namespace b200q
+#include "wq_gemm.cuh"
 
 using namespace b200q;
 
-// Rows from which the tensor-memory GEMM is used.  Measured on a B200 at K=4096, N=28672:
-// the decode kernels take 33 us at 16 rows and 61 us at 32 (one pass, activations shared
-// through shared memory), the GEMM 58 us from 33 to 128 rows; the decode kernel's 64-row
-// pass (98 us) loses to it.
-static constexpr int64_t kGemmRows = 33;
+// Up to this many rows the tensor-core product starts early (its fetch of the weights runs ahead of
+// the kernel before it, as the decode kernels' does).
+static constexpr int64_t kOverlapRows = 64;
+
+// Rows from which the tensor-core product is used.  It takes the same time from 1 to 64 rows; the
+// decode kernels' grows with the rows, less so for groups of 128, which they are specialised for.
+// Decode kernel / tensor-core product, us a launch in a chain on a B200:
+//   groups of 128                 8 rows     9 rows    16 rows    32 rows
+//     4096 -> 4096              4.8/10.6  11.4/10.6  11.8/10.7  18.2/11.9
+//     4096 -> 28672            23.4/31.2  30.5/31.3  31.4/31.3  59.3/31.2
+//     14336 -> 4096            13.6/19.7  26.2/19.7  26.6/19.8  50.9/21.0
+//   other groups                  1 row     3 rows     8 rows    16 rows
+//     32, 2048 -> 2048          5.1/7.4   5.4/7.4    6.4/7.5    8.2/7.5
+//     32, 4096 -> 4096        12.2/10.6 13.7/11.1  17.7/11.2  22.4/11.3
+//     32, 4096 -> 28672       42.9/30.2 49.9/30.3  68.2/30.3 109.7/30.5
+//     64, 4096 -> 6144        11.0/11.9 12.7/12.4  17.1/13.6  23.5/13.7
+//     64, 4096 -> 14336       22.2/17.5 27.0/17.5  35.8/17.6  56.5/17.7
+//     256, 4096 -> 4096         6.1/9.8  7.5/10.3  13.9/10.6  18.6/10.6
+//     256, 4096 -> 14336      15.0/17.3 19.7/17.3  30.3/17.3  49.4/17.4
+static int64_t gemm_rows(int64_t weights, int64_t group) {
+    constexpr int64_t kSome = int64_t(12) << 20, kMany = int64_t(32) << 20;  // weights: 3072 x 4096, 8192 x 4096
+    if (group == 128 || weights < kSome) return 9;
+    if (group < 64) return 1;
+    if (group == 64) return weights < kMany ? 3 : 1;
+    return weights < kMany ? 7 : 3;
+}
 
 extern "C" int32_t b200q_int4_linear_ex(const void* x, const uint8_t* packed, const void* scale,
                                         const uint8_t* zero, void* y, int64_t rows, int64_t in,
                                         int64_t out, int64_t group, int32_t dtype, int32_t flags,
                                         void* stream) {
-    if (rows >= kGemmRows && !(flags & B200Q_SWIGLU_INPUT) && int4_gemm_supports(rows, in, out, group, dtype, x, y))
-        return b200q_int4_gemm(x, packed, scale, zero, y, rows, in, out, group, dtype, stream);
+    if (rows >= gemm_rows(in * out, group) && !(flags & B200Q_SWIGLU_INPUT)) {
+        const int32_t ok = check_int4_args("int4_linear", x, packed, scale, zero, y, rows, in, out, group, dtype);
+        if (ok != B200Q_OK) return ok;
+        const WqProblem p{kWqInt4, x, packed, scale, zero, y, rows, in, out, group, dtype};
+        if (wq_gemm_supports(p))
+            return wq_gemm("int4_linear", p, rows <= kOverlapRows && !(flags & B200Q_NO_OVERLAP),
+                           static_cast<cudaStream_t>(stream));
+    }
     return b200q_int4_gemv_ex(x, packed, scale, zero, y, rows, in, out, group, dtype, flags, stream);
 }
 

@@ -1,5 +1,5 @@
 // tcgen05 / tensor-memory / TMA / mbarrier wrappers shared by the tensor-core GEMM kernels
-// (int4_gemm_sm100.cu: bf16 products of dequantized int4 weights; int8_w8a8.cu: int8 products).
+// (wq_gemm_sm100.cu: 16-bit products of dequantized weights; int8_w8a8.cu: int8 products).
 // Inline PTX for sm_100a only; every mbarrier wait is bounded.
 #pragma once
 
@@ -25,14 +25,17 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
                  : "memory");
 }
+// May suspend the thread until the phase is over, for up to about kSuspendNs: a thread that is
+// asleep takes no issue slots and no shared-memory cycles from the ones it waits for.
+constexpr uint32_t kSuspendNs = 1000000;
 __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
     uint32_t ok;
     asm volatile(
         "{\n.reg .pred p;\n"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n"
         "selp.u32 %0, 1, 0, p;\n}"
         : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity)
+        : "r"(smem_u32(bar)), "r"(parity), "r"(kSuspendNs)
         : "memory");
     return ok != 0;
 }
@@ -41,20 +44,46 @@ __device__ __forceinline__ uint64_t global_timer_ns() {
     asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
     return t;
 }
-// Bounded wait: false (and the error flag set) after about a second.
+// Bounded wait: false (and the error flag set) after about a second.  The clock is not asked for
+// before a wait has lasted a while.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* error, int code) {
-    if (mbar_try_wait(bar, parity)) return true;
-    const uint64_t start = global_timer_ns();
-    for (uint32_t spins = 0;; ++spins) {
+#pragma unroll 1
+    for (int i = 0; i < 32; ++i)
         if (mbar_try_wait(bar, parity)) return true;
-        if ((spins & 1023u) == 1023u) {
-            if (*reinterpret_cast<volatile int*>(error) != 0) return false;  // someone else gave up
-            if (global_timer_ns() - start > 1000000000ull) {
-                atomicCAS(error, 0, code);
-                return false;
-            }
+    const uint64_t start = global_timer_ns();
+#pragma unroll 1
+    for (;;) {
+#pragma unroll 1
+        for (int i = 0; i < 32; ++i)
+            if (mbar_try_wait(bar, parity)) return true;
+        if (*reinterpret_cast<volatile int*>(error) != 0) return false;  // someone else gave up
+        if (global_timer_ns() - start > 1000000000ull) {
+            atomicCAS(error, 0, code);
+            return false;
         }
     }
+}
+// The same for a barrier that threads (or products) of other blocks of the cluster arrive on.
+__device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity, int* error, int code) {
+    uint32_t seen = mbar_wait(bar, parity, error, code);
+    if (seen != 0)  // the phase is over: answered at once
+        asm volatile(
+            "{\n.reg .pred p;\n"
+            "mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+            "selp.u32 %0, 1, 0, p;\n}"
+            : "=r"(seen)
+            : "r"(smem_u32(bar)), "r"(parity)
+            : "memory");
+    return seen != 0;
+}
+__device__ __forceinline__ bool elect_one() {
+    uint32_t leader;
+    asm volatile(
+        "{\n.reg .pred p;\n"
+        "elect.sync _|p, 0xFFFFFFFF;\n"
+        "selp.u32 %0, 1, 0, p;\n}"
+        : "=r"(leader));
+    return leader != 0;
 }
 __device__ __forceinline__ void fence_proxy_async() {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -119,6 +148,44 @@ __device__ __forceinline__ void umma_i8(uint32_t d_tmem, uint64_t a_desc, uint64
         "setp.ne.b32 p, %4, 0;\n"
         "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n}" ::"r"(d_tmem),
         "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+
+// ---- a pair of blocks (cluster of two) as one tensor core: cta_group::2 --------------------------
+// Both blocks hold half of each operand at the same shared-memory offsets; the even block issues.
+__device__ __forceinline__ uint32_t map_to_rank(uint32_t addr, int rank) {
+    uint32_t remote;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(addr), "r"(rank));
+    return remote;
+}
+__device__ __forceinline__ void arrive_cluster(uint32_t remote_bar) {
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(remote_bar) : "memory");
+}
+// A load into this block's own shared memory that counts on a barrier of either block of the pair
+// (`bar`: a shared::cluster address).
+__device__ __forceinline__ void tma_load_2d_pair(void* dst, const CUtensorMap* map, int c0, int c1, uint32_t bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2 "
+        "[%0], [%1, {%2, %3}], [%4];" ::"r"(smem_u32(dst)),
+        "l"(map), "r"(c0), "r"(c1), "r"(bar)
+        : "memory");
+}
+// D[tmem of both] (+)= A[smem of both] . B[smem of both]^T, 256 x N x 32, int8 inputs, int32 accumulate.
+__device__ __forceinline__ void umma_i8_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
+                                             uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n.reg .pred p;\n"
+        "setp.ne.b32 p, %4, 0;\n"
+        "tcgen05.mma.cta_group::2.kind::i8 [%0], %1, %2, %3, p;\n}" ::"r"(d_tmem),
+        "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+// Arrives on this barrier of BOTH blocks when the products issued so far are complete.
+__device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
+    asm volatile(
+        "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
+            smem_u32(bar)),
+        "h"(uint16_t(3))
         : "memory");
 }
 

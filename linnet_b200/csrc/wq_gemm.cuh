@@ -1,0 +1,27 @@
+// Host interface of the tensor-core product of 16-bit activations and quantized weights
+// (wq_gemm_sm100.cu), shared by the int4 and int8 entry points.
+#pragma once
+
+#include "common.cuh"
+
+namespace b200q {
+
+enum WqFormat { kWqInt4 = 0, kWqInt8 = 1 };
+
+struct WqProblem {
+    WqFormat format;
+    const void* x;        // [rows, in] bf16 | f16
+    const void* weight;   // int4: [out, in / 2] u8; int8: [out, in] i8
+    const void* scale;    // int4: [out, in / group] of x's type; int8: f32 [out, in / group]
+    const uint8_t* zero;  // int4: [out, in / group]
+    void* y;              // [rows, out] of x's type
+    int64_t rows, in, out, group;  // group: inputs a scale covers
+    int32_t dtype;
+};
+
+// Whether the kernel takes this problem (at least one row; pointers as the entry points check them).
+bool wq_gemm_supports(const WqProblem& p);
+// Launches it; `overlap`: with programmatic stream serialization.
+int32_t wq_gemm(const char* who, const WqProblem& p, bool overlap, cudaStream_t stream);
+
+}  // namespace b200q

@@ -277,6 +277,17 @@ def w8a16(x: torch.Tensor, weight: torch.Tensor, scale: torch.Tensor, fp8: bool,
     return _eight_bit("w8a16", x, weight, scale, fp8, group, row_block)
 
 
+def w8a16_any_rows(x: torch.Tensor, weight: torch.Tensor, scale: torch.Tensor, group: int) -> bool:
+    """Whether `w8a16` streams this weight once for any number of rows (the tensor-core product):
+    inputs a multiple of 64, one scale a row or groups of 16, 32 or a multiple of 64, and memory
+    that the tiled copies can start at.  Other weights go through the decode kernel in passes of 16
+    rows, which only pays for a few."""
+    return (weight.is_cuda and x.shape[-1] % 64 == 0 and (group in (0, 16, 32) or group % 64 == 0)
+            and x.is_contiguous() and x.data_ptr() % 16 == 0
+            and weight.is_contiguous() and weight.data_ptr() % 16 == 0
+            and scale.dtype == torch.float32 and scale.is_contiguous() and scale.data_ptr() % 16 == 0)
+
+
 def dequantize8(weight: torch.Tensor, scale: torch.Tensor, fp8: bool, group: int, row_block: int,
                 dtype: torch.dtype) -> torch.Tensor:
     """The int8 weight of `gemv8` dequantized to `dtype` (f32 product, one rounding)."""

@@ -6,11 +6,12 @@ per step.  The operand tuples have the reference's members
 (`Int8Operands = (weight, scale_f32, rounded, fast)`, quantized.py:62-66).
 
 Row-count dispatch as the reference's `_weight_only` (quantized.py:90-105): one row goes to
-`gemv8`, up to `TILED_ROWS` rows to `w8a16` (both stream the int8 weight once through the
-decode kernel), more rows dequantize the weight once with `dequantize8` and hand the dense
-product to the library GEMM, which is the reference's own route for that range.  `rounded`
-with more than `FEW_ROWS` rows takes the 8-bit-activation route (`int8_rows` + `int8_mm`,
-quantized.py:187-189).  There is no fallback for CPU tensors.
+`gemv8`, more rows to `w8a16`, whose tensor-core kernel dequantizes the weight inside the product
+at any row count.  Shapes that kernel does not take (`kernels.w8a16_any_rows`) keep the
+reference's route from `TILED_ROWS` rows on: the weight dequantized once with `dequantize8` and
+the dense product handed to the library GEMM.  `rounded` with more than `FEW_ROWS` rows takes the
+8-bit-activation route (`int8_rows` + `int8_mm`, quantized.py:187-189).  There is no fallback for
+CPU tensors.
 """
 
 from __future__ import annotations
@@ -33,7 +34,7 @@ def _weight_only(flat: torch.Tensor, weight: torch.Tensor, scale: torch.Tensor, 
     rows = flat.shape[0]
     if rows == 1:
         return kernels.gemv8(flat, weight, scale, False, group, 1)
-    if rows <= TILED_ROWS:
+    if rows <= TILED_ROWS or kernels.w8a16_any_rows(flat, weight, scale, group):
         return kernels.w8a16(flat, weight, scale, False, group, 1)
     dequantized = kernels.dequantize8(weight, scale, False, group, 1, flat.dtype)
     # f32 accumulation all the way: the library may otherwise add split-K partial sums in the

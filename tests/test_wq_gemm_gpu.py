@@ -1,0 +1,118 @@
+"""The tensor-core product of 16-bit activations and quantized weights at the sizes where it can go
+wrong: one row to several tiles of rows, K that ends in half an item (64 of 128 inputs), one item
+only, ragged N, K split over a cluster, one and two accumulators, every group size it takes, both
+16-bit types, scales at the ends of their range."""
+
+from __future__ import annotations
+
+import pytest
+import torch
+
+from oracle import linear_oracle as lo
+
+pytestmark = pytest.mark.gpu
+
+
+def make_int4(out, depth, group, dtype, gen, magnitude=1.0):
+    packed = torch.randint(0, 256, (out, depth // group, group // 2), generator=gen, dtype=torch.uint8)
+    scale = ((torch.rand(out, depth // group, generator=gen) * 0.9 + 0.1) * magnitude).to(dtype)
+    zero = torch.randint(0, 16, (out, depth // group), generator=gen, dtype=torch.uint8)
+    return packed, scale, zero
+
+
+def make_int8(out, depth, group, gen):
+    weight = torch.randint(-128, 128, (out, depth), generator=gen, dtype=torch.int8)
+    return weight, torch.rand(out, depth // (group or depth), generator=gen) * 0.01 + 1e-4
+
+
+def check(got, x, w):
+    """Against the f64 product of the same rounded weights: one rounding to the result's type plus
+    f32 sums of `depth` products, each addition off by at most an ulp (2^-23, the tensor cores
+    truncate) of the sum of magnitudes."""
+    exact = x.double() @ w.double().T
+    size = x.double().abs() @ w.double().abs().T
+    ulp = 2.0 ** -8 if got.dtype == torch.bfloat16 else 2.0 ** -11
+    bound = ulp * exact.abs() + x.shape[1] * 2.0 ** -23 * size + 1e-30
+    assert bool(((got.double().cpu() - exact).abs() <= 1.01 * bound).all())
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("group", [16, 32, 64, 128, 384])
+def test_int4_weights_are_exact(dtype, group):
+    """The identity times W^T is W bit for bit, also where the fast conversion's power of two would
+    leave the type's range (scales near its largest value) and for subnormal scales."""
+    from linnet_b200 import kernels
+
+    depth, out = 768, 200
+    gen = torch.Generator().manual_seed(group)
+    top = 2.0 ** 124 if dtype == torch.bfloat16 else 2000.0  # 15 times the scale is still finite
+    for magnitude in (0.01, top, 2.0 ** -130 if dtype == torch.bfloat16 else 2.0 ** -20):
+        packed, scale, zero = make_int4(out, depth, group, dtype, gen, magnitude)
+        got = kernels.int4_linear(torch.eye(depth, dtype=dtype).cuda(), packed.cuda(), scale.cuda(), zero.cuda())
+        want = lo.int4_weight(packed, scale, zero, dtype)
+        assert torch.equal(got.t().cpu().float(), want.float())
+
+
+# (rows, depth, out): the plans these reach are one item; a last item of half; a K split of four;
+# two tiles a block with two accumulators; two blocks of rows a tile; one accumulator (rows 200, 256);
+# several tiles of rows with a ragged last one
+SHAPES = [(1, 64, 128), (9, 128, 100), (17, 192, 1000), (33, 4160, 130), (64, 4096, 512), (16, 1024, 28680),
+          (100, 320, 20000), (200, 448, 3000), (256, 1088, 4096), (257, 640, 5000), (1000, 256, 9001)]
+
+
+@pytest.mark.parametrize(("rows", "depth", "out"), SHAPES)
+@pytest.mark.parametrize(("group", "dtype"), [(64, torch.bfloat16), (32, torch.float16), (16, torch.bfloat16)])
+def test_int4_product(rows, depth, out, group, dtype):
+    from linnet_b200 import kernels
+
+    gen = torch.Generator().manual_seed(rows + depth + out + group)
+    packed, scale, zero = make_int4(out, depth, group, dtype, gen, 0.02)
+    x = torch.randn(rows, depth, generator=gen).to(dtype)
+    got = kernels.int4_linear(x.cuda(), packed.cuda(), scale.cuda(), zero.cuda())
+    check(got, x, lo.int4_weight(packed, scale, zero, dtype))
+
+
+@pytest.mark.parametrize(("rows", "depth", "out"), SHAPES)
+@pytest.mark.parametrize(("group", "dtype"), [(0, torch.bfloat16), (32, torch.bfloat16), (64, torch.float16)])
+def test_int8_product(rows, depth, out, group, dtype):
+    from linnet_b200 import quantized
+
+    if rows <= 2 and not group:
+        pytest.skip("one or two rows with one scale a row run another kernel")
+    gen = torch.Generator().manual_seed(rows + depth + out + group)
+    weight, scale = make_int8(out, depth, group, gen)
+    x = torch.randn(rows, depth, generator=gen).to(dtype)
+    if group:
+        got = quantized.int8_group_linear(x.cuda(), quantized.int8_group_operands(weight.cuda(), scale.cuda()), None)
+    else:
+        got = quantized.int8_linear(x.cuda(), quantized.int8_operands(weight.cuda(), scale.cuda(), 0), None)
+    check(got, x, lo.int8_weight(weight, scale if group else scale.reshape(-1), dtype))
+
+
+def test_slow_scales_do_not_outrun_the_weights():
+    """Groups of 32 over a wide weight, many launches: the scattered scale loads keep the load unit
+    busy while the stages of packed weights are handed back (results are the same every time)."""
+    from linnet_b200 import _lib, kernels
+
+    gen = torch.Generator().manual_seed(2)
+    packed, scale, zero = (t.cuda() for t in make_int4(14336, 4096, 32, torch.bfloat16, gen, 0.02))
+    x = torch.randn(300, 4096, generator=gen).to(torch.bfloat16).cuda()
+    first = kernels.int4_linear(x, packed, scale, zero)
+    check(first[:, :256], x.cpu(), lo.int4_weight(packed[:256].cpu(), scale[:256].cpu(), zero[:256].cpu(), torch.bfloat16))
+    for _ in range(10):
+        assert torch.equal(kernels.int4_linear(x, packed, scale, zero), first)
+    assert _lib.load().b200q_int4_gemm_status() == 0
+
+
+def test_unaligned_activations_keep_the_library_route():
+    """int8 rows that do not start on 16 bytes: what the tiled copies cannot read is still taken."""
+    from linnet_b200 import kernels, quantized
+
+    gen = torch.Generator().manual_seed(4)
+    weight, scale = make_int8(256, 512, 0, gen)
+    x = torch.randn(100 * 512 + 1, generator=gen).to(torch.bfloat16)
+    inner = x.cuda()[1:].view(100, 512)
+    operands = quantized.int8_operands(weight.cuda(), scale.cuda(), 0)
+    assert not kernels.w8a16_any_rows(inner, operands[0], operands[1], 0)
+    got = quantized.int8_linear(inner, operands, None)
+    check(got, x[1:].view(100, 512), lo.int8_weight(weight, scale.reshape(-1), torch.bfloat16))
