@@ -32,10 +32,11 @@ def _int4_weight(raw: torch.Tensor, scale: torch.Tensor, zero: torch.Tensor) -> 
 def _int4_linear(x, packed, bias, raw, scale, zero):
     """Same signature as the generated helper; every row count goes to
     `linnet::int4_linear`, which picks the decode kernel or the tensor-memory GEMM."""
-    flat = x.reshape(-1, x.shape[-1])
+    flat = x if x.dim() == 2 else x.reshape(-1, x.shape[-1])
     if len(packed) == 3:
         y = kernels.int4_linear(flat, packed[0], packed[1], packed[2])
     else:
         y = kernels.int4_linear(flat, raw, scale, zero)
-    y = y.reshape(*x.shape[:-1], y.shape[-1])
+    if flat is not x:
+        y = y.reshape(*x.shape[:-1], y.shape[-1])
     return y if bias is None else y + bias

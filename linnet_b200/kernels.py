@@ -29,24 +29,30 @@ def _code(dtype: torch.dtype, who: str) -> int:
 
 
 def _on_gpu(who: str, *tensors: torch.Tensor) -> torch.device:
-    device = tensors[0].device
+    index = tensors[0].get_device()  # -1 off the GPU; cheaper to compare than `device` objects
     for t in tensors:
-        if not t.is_cuda or t.device != device:
+        if not t.is_cuda or t.get_device() != index:
             raise RuntimeError(
                 f"{who}: every tensor must be on one CUDA device (there is no CPU path in "
                 f"this build); got {[str(t.device) for t in tensors]}")
-    return device
+    return tensors[0].device
+
+
+# PyTorch's own accessors, without the Stream object and the initialisation check that
+# `torch.cuda.current_stream` and `current_device` go through: a one-row call is bound by its host path.
+_raw_stream = torch._C._cuda_getCurrentRawStream
+_current_device = torch._C._cuda_getDevice
 
 
 def _stream(device: torch.device) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+    return _raw_stream(device.index)
 
 
 class _Device:
     """Makes `device` current for the launch when it is not already."""
 
     def __init__(self, device: torch.device) -> None:
-        self.guard = None if device.index == torch.cuda.current_device() else torch.cuda.device(device)
+        self.guard = None if device.index == _current_device() else torch.cuda.device(device)
 
     def __enter__(self) -> None:
         if self.guard is not None:

@@ -49,7 +49,8 @@ def _weight_only(flat: torch.Tensor, weight: torch.Tensor, scale: torch.Tensor, 
 
 
 def _finish(x: torch.Tensor, y: torch.Tensor, bias: torch.Tensor | None) -> torch.Tensor:
-    y = y.reshape(*x.shape[:-1], y.shape[-1])
+    if x.dim() != 2:
+        y = y.reshape(*x.shape[:-1], y.shape[-1])
     return y if bias is None else y + bias
 
 
@@ -68,7 +69,7 @@ def int8_operands(weight: torch.Tensor, scale: torch.Tensor, rounded: int) -> In
 def int8_linear(x: torch.Tensor, operands: Int8Operands, bias: torch.Tensor | None) -> torch.Tensor:
     weight, scale, rounded, _fast = operands
     _require(x, "int8_linear")
-    flat = x.reshape(-1, x.shape[-1])
+    flat = x if x.dim() == 2 else x.reshape(-1, x.shape[-1])
     if rounded and flat.shape[0] > FEW_ROWS and kernels.int8_mm_available(weight):
         q, row_scale = kernels.int8_rows(flat)
         y = kernels.int8_mm(q, weight, row_scale, scale, flat.dtype)
@@ -89,5 +90,5 @@ def int8_group_linear(x: torch.Tensor, operands: Int8GroupOperands,
                       bias: torch.Tensor | None) -> torch.Tensor:
     weight, scale, group, _fast = operands
     _require(x, "int8_group_linear")
-    flat = x.reshape(-1, x.shape[-1])
+    flat = x if x.dim() == 2 else x.reshape(-1, x.shape[-1])
     return _finish(x, _weight_only(flat, weight, scale, group), bias)
