@@ -232,13 +232,23 @@ __device__ __forceinline__ void tmem_store_32(uint32_t taddr, const uint32_t (&v
         : "memory");
 }
 // 16 columns of this thread's lane.
-__device__ __forceinline__ void tmem_load_16(uint32_t (&v)[16], uint32_t taddr) {
+__device__ __forceinline__ void tmem_ask_16(uint32_t (&v)[16], uint32_t taddr) {  // v is there after tmem_wait()
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
         : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
           "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
         : "r"(taddr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_wait(uint32_t (&v)[16]) {  // (v passes through: no use of it moves above)
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]),
+                   "+r"(v[8]), "+r"(v[9]), "+r"(v[10]), "+r"(v[11]), "+r"(v[12]), "+r"(v[13]), "+r"(v[14]), "+r"(v[15])
+                 :
+                 : "memory");
+}
+__device__ __forceinline__ void tmem_load_16(uint32_t (&v)[16], uint32_t taddr) {
+    tmem_ask_16(v, taddr);
+    tmem_wait(v);
 }
 // D[tmem] (+)= A[tmem] . B[smem]^T, 128 x N x 16, 16-bit inputs, f32 accumulate.
 __device__ __forceinline__ void umma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
@@ -543,29 +553,49 @@ wq_gemm_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant_
                         tc_fence_after();
                     }
                     const int n = (tile / a.m_tiles * R + r) * kTileRows + warp * 32 + lane;
-#pragma unroll 1
-                    for (int c0 = 0; c0 < nx; c0 += 16) {
-                        if (c0 >= live) break;
-                        uint32_t v[16];
-                        sums(v, r, c0);
+                    auto store = [&](const uint32_t (&v)[16], int c0) {  // 16 rows of Y, this lane's column
                         uint16_t* dst = a.y + size_t(m0 + c0) * a.N + n;
                         if (a.pairs) {
                             // lanes 2i and 2i+1 trade values, so that each stores a pair of
                             // columns of one row of Y: 4-byte stores, two rows an instruction
                             const int odd = lane & 1;
+                            dst += odd ? ptrdiff_t(a.N) - 1 : 0;
 #pragma unroll
                             for (int j = 0; j < 16; j += 2) {
                                 const uint32_t mine = odd ? v[j + 1] : v[j];
                                 const uint32_t other = __shfl_xor_sync(0xFFFFFFFFu, odd ? v[j] : v[j + 1], 1);
                                 const uint32_t packed = odd ? H::pack(__uint_as_float(other), __uint_as_float(mine))
                                                             : H::pack(__uint_as_float(mine), __uint_as_float(other));
-                                if (c0 + j + odd < live && n < a.N)
-                                    *reinterpret_cast<uint32_t*>(dst + size_t(j + odd) * a.N - odd) = packed;
+                                if (c0 + j + odd < live && n < a.N) *reinterpret_cast<uint32_t*>(dst) = packed;
+                                dst += 2 * size_t(a.N);
                             }
                         } else {
 #pragma unroll
                             for (int j = 0; j < 16; ++j)
                                 if (c0 + j < live && n < a.N) dst[size_t(j) * a.N] = H::from_float(__uint_as_float(v[j]));
+                        }
+                    };
+                    if (both) {
+#pragma unroll 1
+                        for (int c0 = 0; c0 < live; c0 += 16) {
+                            uint32_t v[16];
+                            sums(v, r, c0);
+                            store(v, c0);
+                        }
+                    } else {
+                        // the next 16 columns are on their way while these are stored
+                        const uint32_t from = lanes + uint32_t((R == 1 ? first_sum : r) * nx);
+                        uint32_t v[16], u[16];
+                        tmem_ask_16(v, from);
+#pragma unroll 1
+                        for (int c0 = 0; c0 < live; c0 += 32) {
+                            tmem_wait(v);
+                            if (c0 + 16 < live) tmem_ask_16(u, from + uint32_t(c0 + 16));
+                            store(v, c0);
+                            if (c0 + 16 >= live) break;
+                            tmem_wait(u);
+                            if (c0 + 32 < live) tmem_ask_16(v, from + uint32_t(c0 + 32));
+                            store(u, c0 + 16);
                         }
                     }
                     tc_fence_before();
