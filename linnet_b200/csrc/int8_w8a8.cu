@@ -16,6 +16,8 @@
 // One persistent block per multiprocessor walks over the 128 x BN tiles; the accumulators are
 // double-buffered so a tile's epilogue overlaps the next tile's products.  Every mbarrier
 // wait is bounded (shared with the int4 GEMM: b200q_int4_gemm_status() reports an expiry).
+#include <atomic>
+
 #include "mma.cuh"
 #include "umma.cuh"
 
@@ -121,6 +123,44 @@ struct Pipe8 {
     uint32_t tmem_base;
 };
 
+// One finished accumulator: this thread's row m (a lane of tensor memory), bn columns from n0.
+__device__ __forceinline__ void store_tile(const MmArgs& a, uint32_t taddr, int m, int n0, int bn) {
+    const float xs = m < a.M ? __ldg(a.x_scale + m) : 0.0f;
+#pragma unroll 1
+    for (int c0 = 0; c0 < bn; c0 += 32) {
+        uint32_t v[32];
+        tmem_load_32(v, taddr + c0);  // (past bn: not stored)
+        if (m < a.M) {
+            uint16_t* dst = a.y + size_t(m) * a.N + n0 + c0;
+            const int live = min(min(bn - c0, a.N - n0 - c0), 32);  // columns of this chunk that exist
+            uint16_t out[32];
+#pragma unroll
+            for (int j = 0; j < 32; ++j) {
+                const int n = n0 + c0 + j;
+                const float ws = j < live ? __ldg(a.w_scale + n) : 0.0f;
+                const float r = __fmul_rn(__fmul_rn(float(int32_t(v[j])), xs), ws);
+                out[j] = a.f16 ? Half16<__half>::from_float(r) : Half16<__nv_bfloat16>::from_float(r);
+            }
+            if (a.vec) {  // bn, n0 and N are multiples of 8: 16-byte pieces are whole or absent
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    if (8 * j >= live) break;
+                    uint4 o;
+                    o.x = uint32_t(out[8 * j + 0]) | (uint32_t(out[8 * j + 1]) << 16);
+                    o.y = uint32_t(out[8 * j + 2]) | (uint32_t(out[8 * j + 3]) << 16);
+                    o.z = uint32_t(out[8 * j + 4]) | (uint32_t(out[8 * j + 5]) << 16);
+                    o.w = uint32_t(out[8 * j + 6]) | (uint32_t(out[8 * j + 7]) << 16);
+                    reinterpret_cast<uint4*>(dst)[j] = o;
+                }
+            } else {
+#pragma unroll
+                for (int j = 0; j < 32; ++j)
+                    if (j < live) dst[j] = out[j];
+            }
+        }
+    }
+}
+
 template <int BN>
 __global__ void __launch_bounds__(kThreads, 1)
 int8_mm_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CUtensorMap w_map,
@@ -216,40 +256,7 @@ int8_mm_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant_
             if (!ok) break;
             tc_fence_after();
             const int m = m0 + warp * 32 + lane;
-            const float xs = m < a.M ? __ldg(a.x_scale + m) : 0.0f;
-#pragma unroll 1
-            for (int c0 = 0; c0 < bn; c0 += 32) {
-                uint32_t v[32];
-                tmem_load_32(v, tmem + (uint32_t(warp * 32) << 16) + buf * BN + c0);  // (past bn: not stored)
-                if (m < a.M) {
-                    uint16_t* dst = a.y + size_t(m) * a.N + n0 + c0;
-                    const int live = min(min(bn - c0, a.N - n0 - c0), 32);  // columns of this chunk that exist
-                    uint16_t out[32];
-#pragma unroll
-                    for (int j = 0; j < 32; ++j) {
-                        const int n = n0 + c0 + j;
-                        const float ws = j < live ? __ldg(a.w_scale + n) : 0.0f;
-                        const float r = __fmul_rn(__fmul_rn(float(int32_t(v[j])), xs), ws);
-                        out[j] = a.f16 ? Half16<__half>::from_float(r) : Half16<__nv_bfloat16>::from_float(r);
-                    }
-                    if (a.vec) {  // bn, n0 and N are multiples of 8: 16-byte pieces are whole or absent
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            if (8 * j >= live) break;
-                            uint4 o;
-                            o.x = uint32_t(out[8 * j + 0]) | (uint32_t(out[8 * j + 1]) << 16);
-                            o.y = uint32_t(out[8 * j + 2]) | (uint32_t(out[8 * j + 3]) << 16);
-                            o.z = uint32_t(out[8 * j + 4]) | (uint32_t(out[8 * j + 5]) << 16);
-                            o.w = uint32_t(out[8 * j + 6]) | (uint32_t(out[8 * j + 7]) << 16);
-                            reinterpret_cast<uint4*>(dst)[j] = o;
-                        }
-                    } else {
-#pragma unroll
-                        for (int j = 0; j < 32; ++j)
-                            if (j < live) dst[j] = out[j];
-                    }
-                }
-            }
+            store_tile(a, tmem + (uint32_t(warp * 32) << 16) + buf * BN, m, n0, bn);
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&pipe->acc_empty[buf]);
@@ -262,6 +269,173 @@ int8_mm_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant_
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(S::kTmemColumns)
                      : "memory");
     }
+}
+
+// ---- int8_mm on pairs of blocks ----------------------------------------------------------------
+// A tile of 256 x bn as ONE product of a pair of multiprocessors (cta_group::2): each block loads
+// its own 128 rows of x and HALF of the tile's rows of W, so that per product a multiprocessor
+// reads 32 + bn / 8 B a clock of shared memory instead of 32 * (128 + bn) * 2 / bn: the one-block
+// kernel above, which wants about 200 B a clock (operands and TMA writes) of the 128 there are, is
+// bound by that.  In a chain of launches, one-block -> pair, us: 2048 x 4096 -> 14336 95.9 -> 85.9
+// (2.8 POP/s, 0.88 of twice the bf16 rate a library GEMM holds here), 2048 x 14336 -> 4096 90.5 ->
+// 80.2, 1024 x 14336 -> 4096 68.3 -> 44.6, 256 x 4096 -> 4096 14.1 -> 11.3.  Stages of 256 inputs
+// (half as many waits) were 2 to 15 % slower: fewer, larger stages hide less of the loads' latency.
+constexpr int kPairStages = 6, kPairStageBytes = 2 * 128 * kBK;
+constexpr size_t kPairSmem = size_t(kPairStages) * kPairStageBytes + 1024 + 256;
+
+struct PipePair {
+    uint64_t full[kPairStages];   // of the even block: both blocks' TMA bytes landed
+    uint64_t empty[kPairStages];  // of each block: the products that read the stage completed
+    uint64_t acc_full[2];         // of each block: all products of a tile completed
+    uint64_t acc_empty[2];        // of the even block: both epilogues drained the accumulator
+    uint32_t tmem_base;
+};
+
+__global__ void __launch_bounds__(kThreads, 1)
+int8_mm_pair_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CUtensorMap w_map,
+                    const MmArgs a, int* error) {
+    extern __shared__ __align__(1024) uint8_t smem_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    PipePair* pipe = reinterpret_cast<PipePair*>(smem + kPairStages * kPairStageBytes);
+    const int warp = __shfl_sync(0xFFFFFFFFu, int(threadIdx.x) / 32, 0), lane = threadIdx.x % 32;
+    const int rank = int(blockIdx.x) & 1, pair = int(blockIdx.x) >> 1, pairs = int(gridDim.x) >> 1;
+    const int tiles = a.m_tiles * a.n_tiles, ksteps = a.K / kBK, bn = a.bn;
+    const uint32_t b_at = 128 * kBK;  // W's half behind the rows of x
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < kPairStages; ++s) {
+            mbar_init(&pipe->full[s], 1);
+            mbar_init(&pipe->empty[s], 1);
+        }
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(&pipe->acc_full[b], 1);
+            mbar_init(&pipe->acc_empty[b], 2 * kEpilogueWarps);
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == kMmaWarp) {  // in both blocks
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                         smem_u32(&pipe->tmem_base)),
+                     "r"(512u)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync();  // the other block's barriers and tensor memory are there
+    tc_fence_after();
+    const uint32_t tmem = pipe->tmem_base;
+    pdl_wait();  // the rounded activations come from the kernel ahead of this one
+    pdl_launch_dependents();
+
+    if (warp == kTmaWarp) {
+        if (lane == 0) {
+            int s = 0;
+            uint32_t lap = 0;
+            bool ok = true;
+            for (int tile = pair; tile < tiles && ok; tile += pairs) {
+                const int m0 = (tile % a.m_tiles) * 256 + rank * 128, n0 = (tile / a.m_tiles) * bn + rank * (bn / 2);
+                for (int ks = 0; ks < ksteps && ok; ++ks) {
+                    if (lap > 0) ok = mbar_wait(&pipe->empty[s], (lap - 1) & 1, error, 11);
+                    if (!ok) break;
+                    uint8_t* dst = smem + s * kPairStageBytes;
+                    const uint32_t bar = map_to_rank(smem_u32(&pipe->full[s]), 0);
+                    if (rank == 0) mbar_expect_tx(&pipe->full[s], uint32_t(2 * (128 + bn / 2) * kBK));
+                    tma_load_2d_pair(dst, &x_map, ks * kBK, m0, bar);
+                    tma_load_2d_pair(dst + b_at, &w_map, ks * kBK, n0, bar);
+                    if (++s == kPairStages) s = 0, ++lap;
+                }
+            }
+            // given up: the copies in flight of both blocks count on the even block's barriers
+            for (int i = 0; i < kPairStages && !ok && rank == 0; ++i)
+                if (lap > 0 || i < s) mbar_wait(&pipe->full[i], (i < s ? lap : lap - 1) & 1, error, 15);
+        }
+    } else if (warp == kMmaWarp) {
+        if (rank == 0) {
+            // int32 accumulator, signed 8-bit A and B, both K-major, M = 256, N = bn
+            const uint32_t idesc = (2u << 4) | (1u << 7) | (1u << 10) | (uint32_t(bn >> 3) << 17) | (uint32_t(256 >> 4) << 24);
+            const bool leader = elect_one();
+            const uint64_t desc = smem_desc(smem_u32(smem));
+            uint32_t t = 0, phase = 0;
+            int s = 0;
+            bool ok = true;
+            for (int tile = pair; tile < tiles && ok; tile += pairs, ++t) {
+                const uint32_t buf = t & 1;
+                if (t >= 2) ok = __all_sync(0xFFFFFFFFu, mbar_wait_cluster(&pipe->acc_empty[buf], ((t / 2) - 1) & 1, error, 12));
+                for (int ks = 0; ks < ksteps && ok; ++ks) {
+                    ok = __all_sync(0xFFFFFFFFu, mbar_wait_cluster(&pipe->full[s], phase, error, 13));
+                    if (!ok) break;
+                    tc_fence_after();
+                    if (leader) {
+                        const uint64_t at = desc + uint32_t(s) * (kPairStageBytes >> 4);
+#pragma unroll
+                        for (int kk = 0; kk < kBK / 32; ++kk)
+                            umma_i8_pair(tmem + buf * 256, at + 2 * kk, at + (b_at >> 4) + 2 * kk, idesc,
+                                         kk > 0 ? 1u : uint32_t(ks > 0));
+                        umma_commit_pair(&pipe->empty[s]);
+                    }
+                    __syncwarp();
+                    if (++s == kPairStages) s = 0, phase ^= 1;
+                }
+                if (leader && ok) umma_commit_pair(&pipe->acc_full[buf]);
+                __syncwarp();
+            }
+        }
+    } else {
+        uint32_t t = 0;
+        bool ok = true;
+        for (int tile = pair; tile < tiles && ok; tile += pairs, ++t) {
+            const int m0 = (tile % a.m_tiles) * 256 + rank * 128, n0 = (tile / a.m_tiles) * bn;
+            const uint32_t buf = t & 1;
+            ok = __all_sync(0xFFFFFFFFu, mbar_wait_cluster(&pipe->acc_full[buf], (t / 2) & 1, error, 14));
+            if (!ok) break;
+            tc_fence_after();
+            store_tile(a, tmem + (uint32_t(warp * 32) << 16) + buf * 256, m0 + warp * 32 + lane, n0, bn);
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) arrive_cluster(map_to_rank(smem_u32(&pipe->acc_empty[buf]), 0));
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync();  // nobody leaves, or gives its tensor memory back, while the other may still use it
+    if (warp == kMmaWarp) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
+    }
+}
+
+constexpr double kPairFixed = 64, kSingle = 1.2;
+
+void pair_config(cudaLaunchConfig_t* config, cudaLaunchAttribute* attr, int pairs) {
+    ensure_dynamic_smem(reinterpret_cast<const void*>(int8_mm_pair_kernel), kPairSmem);
+    config->gridDim = dim3(unsigned(2 * pairs));
+    config->blockDim = dim3(kThreads);
+    config->dynamicSmemBytes = kPairSmem;
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    config->attrs = attr;
+    config->numAttrs = 1;
+}
+
+// Pairs of blocks the device holds at a time (0: none); asked for once per device.
+int resident_pairs() {
+    static std::atomic<int> cached[64];
+    int device = 0;
+    if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) return 0;
+    int count = cached[device].load(std::memory_order_relaxed);
+    if (count == 0) {
+        cudaLaunchConfig_t config = {};
+        cudaLaunchAttribute attr[1];
+        pair_config(&config, attr, 1);
+        if (cudaOccupancyMaxActiveClusters(&count, int8_mm_pair_kernel, &config) != cudaSuccess || count <= 0) {
+            cudaGetLastError();
+            return 0;
+        }
+        cached[device].store(count, std::memory_order_relaxed);
+    }
+    return count;
 }
 
 int32_t make_map(CUtensorMap* map, const void* base, int64_t rows, int64_t depth, int box_rows, const char* who) {
@@ -315,6 +489,46 @@ extern "C" int32_t b200q_int8_mm(const int8_t* xq, const int8_t* w, const float*
     B200Q_REQUIRE(error != nullptr, "int8_mm: no status word on this device");
     const int sms = sm_count();
     const int m_tiles = int((rows + kBM - 1) / kBM);
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    CUtensorMap x_map, w_map;
+    int32_t status = make_map(&x_map, xq, rows, in, kBM, "int8_mm");
+    if (status != B200Q_OK) return status;
+    // Pairs of blocks on 256-row tiles, where they need no more rounds of tiles than pay: a pair's
+    // tile takes about as long as bn + kPairFixed columns, the one-block kernel's 128-row tile
+    // kSingle times as much a column (300 rows x 4096 -> 28672, which fill three 128-row tiles and
+    // two 256-row ones: 46.8 us against a pair's 49.6; 400 rows: 57.2 against 51.9).
+    const int pairs = resident_pairs();
+    if (rows > kBM && pairs > 0) {
+        const int m_pairs = int((rows + 255) / 256);
+        int bn = 0;
+        double best = 0.0;
+        for (int width = 256; width >= 128; width -= 32) {
+            const int64_t count = int64_t(m_pairs) * ((out + width - 1) / width);
+            const double cost = double(width + kPairFixed) * double((count + pairs - 1) / pairs);
+            if (bn == 0 || cost < best) bn = width, best = cost;
+        }
+        double single = 0.0;
+        for (int width = 256; width >= 128; width -= 16) {
+            const int64_t count = int64_t(m_tiles) * ((out + width - 1) / width);
+            const double cost = double(width + 64) * double((count + sms - 1) / sms) * kSingle;
+            if (width == 256 || cost < single) single = cost;
+        }
+        if (best <= single) {
+            status = make_map(&w_map, w, out, in, bn / 2, "int8_mm");
+            if (status != B200Q_OK) return status;
+            MmArgs a{x_scale, w_scale, static_cast<uint16_t*>(y), int(rows), int(in), int(out), m_pairs,
+                     int((out + bn - 1) / bn), bn, dtype == B200Q_F16 ? 1 : 0, (out % 8 == 0 && aligned(y, 16)) ? 1 : 0};
+            const int tiles = a.m_tiles * a.n_tiles;
+            cudaLaunchConfig_t config = {};
+            cudaLaunchAttribute attr[2];
+            pair_config(&config, attr, tiles < pairs ? tiles : pairs);
+            attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+            attr[1].val.programmaticStreamSerializationAllowed = 1;
+            config.numAttrs = 2;
+            config.stream = s;
+            return launch_status("int8_mm", cudaLaunchKernelEx(&config, int8_mm_pair_kernel, x_map, w_map, a, error));
+        }
+    }
     // 256-wide tiles halve the traffic of x when there are enough tiles to go round
     const bool wide = int64_t(m_tiles) * ((out + 255) / 256) >= sms;
     // ... and of the wide tiles (144 to 256 rows of W in steps of 16) the width that fills the
@@ -329,16 +543,12 @@ extern "C" int32_t b200q_int8_mm(const int8_t* xq, const int8_t* w, const float*
             if (width == 256 || cost < best) bn = width, best = cost;
         }
     }
-    CUtensorMap x_map, w_map;
-    int32_t status = make_map(&x_map, xq, rows, in, kBM, "int8_mm");
-    if (status != B200Q_OK) return status;
     status = make_map(&w_map, w, out, in, bn, "int8_mm");
     if (status != B200Q_OK) return status;
     MmArgs a{x_scale, w_scale, static_cast<uint16_t*>(y), int(rows), int(in), int(out), m_tiles,
              int((out + bn - 1) / bn), bn, dtype == B200Q_F16 ? 1 : 0, (out % 8 == 0 && aligned(y, 16)) ? 1 : 0};
     const int tiles = a.m_tiles * a.n_tiles;
     const int grid = tiles < sms ? tiles : sms;
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
     cudaError_t err;
     if (wide) {
         ensure_dynamic_smem(reinterpret_cast<const void*>(int8_mm_kernel<256>), Shape8<256>::kSmem);
