@@ -1,23 +1,25 @@
 // int8 per-channel decode kernel for one or two activation rows: the structure of the int4
 // kernel of int4_gemv_tma.cuh (one block per multiprocessor, the weights brought by the TMA
 // unit into a ring of shared-memory stages, a producer thread, consumer warps that never issue
-// a weight load) with each weight byte taken as two 4-bit planes.
+// a weight load).
 //
-//   u = w + 128 = 16 h + l  (one XOR per word makes the byte unsigned)
-//   y[m, n] = scale[n] * ( sum_k x[m, k] (magic + l[n, k]) + sum_k 16 x[m, k] (magic + h[n, k])
-//                          - (17 magic + 128) X[m] ),      X[m] = sum_k x[m, k]
+//   y[m, n] = scale[n] * sum_k x[m, k] w[n, k]
 //
-// magic + nibble (128 + q in bf16, 1024 + q in f16) is what one LOP3 makes of a pair of nibbles,
-// and it is exact; 16 x is exact in the 16-bit type (a power of two); the products are exact in
-// f32.  So the same seven integer instructions a 32-bit word that unpack eight int4 weights
-// unpack four int8 weights here, and the kernel streams int8 bytes at the rate the int4 kernel
-// streams int4 bytes.  The per-row scale multiplies the finished sum, as in the kernel this one
+// A byte u = w + 128 (one XOR per word makes the bytes unsigned) becomes a 16-bit float with one
+// byte permute and one multiply-add per pair: in bf16 the byte in the low bits reads as u * 2^-133,
+// times 2^127 less 2 is (u - 128) / 64, exact in 8 bits; in f16 0x6400 | u is 1024 + u, less 1152 is
+// w.  Five instructions (three of the integer pipe) and one MMA a word of four weights.  Before, a
+// byte was taken as two 4-bit planes: seven integer instructions and two MMAs a word, and sums of
+// (128 + q) that a correction had to bring back; 18.0 us a launch at 4096 -> 14336 against 16.3 now,
+// two rows at 14336 -> 4096 30.2 against 16.6.
+// The per-row scale multiplies the finished sum, as in the kernel this one
 // relieves for one and two rows (int8_gemv.cu), and as linnet::gemv8 does
 // (python/linnet/src/linnet/torch/kernels.py:336-434).
 //
 // A k-block is 64 inputs (64 bytes of a row); an item is 16 rows x KB k-blocks, one 3-D TMA
-// box landing as [KB][16 rows][64 bytes].  The activations are staged once per block as B
-// fragments: for the four inputs of a word, (x0, x2), 16 (x0, x2), (x1, x3), 16 (x1, x3).
+// box landing as [KB][16 rows][64 bytes].  A lane's 16 bytes of a row are its 16 inputs of the
+// k-block, so the activations are staged once per block as they are: 32 bytes a lane are the B
+// fragments of the four words.
 #pragma once
 
 #include <cuda.h>
@@ -42,9 +44,8 @@ struct Tma8Args {
 };
 
 struct Tma8Layout {
-    uint32_t bars, xs, xsum, total;
+    uint32_t bars, xs, total;
     uint32_t xrow;  // bytes of one activation row in xs
-    int xpairs;     // pairs of rows in xsum
 };
 template <int WARPS, int KB>
 __host__ __device__ inline Tma8Layout tma8_layout(int M, int K, int stages) {
@@ -52,18 +53,28 @@ __host__ __device__ inline Tma8Layout tma8_layout(int M, int K, int stages) {
     const int kblocks = K / 64;
     l.bars = uint32_t(stages) * (KB * 1024);
     l.xs = (l.bars + uint32_t(stages + 2 * WARPS) * 8 + 127u) & ~127u;
-    l.xrow = uint32_t(kblocks) * 256 + (M > 1 ? 64 : 0);
-    l.xpairs = (M + 1) / 2;
-    l.xsum = l.xs + uint32_t(M) * l.xrow;
-    l.total = l.xsum + uint32_t(l.xpairs) * kblocks * 8;
+    l.xrow = uint32_t(kblocks) * 128 + (M > 1 ? 16 : 0);
+    l.total = l.xs + uint32_t(M) * l.xrow;
     return l;
+}
+
+// Two int8 weights (bytes of u = w + 128 that `selector` picks) as a pair: w in f16, w / 64 in bf16.
+__device__ __forceinline__ uint32_t widen8(uint32_t u, bool second, __half) {
+    const uint32_t v = __byte_perm(u, 0x64646464u, second ? 0x4342u : 0x4140u), bias = 0x64806480u;  // 1152
+    const __half2 r = __hsub2(*reinterpret_cast<const __half2*>(&v), *reinterpret_cast<const __half2*>(&bias));
+    return *reinterpret_cast<const uint32_t*>(&r);
+}
+__device__ __forceinline__ uint32_t widen8(uint32_t u, bool second, __nv_bfloat16) {
+    const uint32_t v = __byte_perm(u, 0u, second ? 0x4342u : 0x4140u);
+    uint32_t r;
+    asm("fma.rn.bf16x2 %0, %1, %2, %3;" : "=r"(r) : "r"(v), "r"(0x7F007F00u), "r"(0xC000C000u));  // 2^127, -2
+    return r;
 }
 
 template <typename T, int WARPS, int KB>
 __global__ void __launch_bounds__((WARPS + 1) * 32, 1)
 int8_gemv_tma_kernel(const __grid_constant__ CUtensorMap wmap, const Tma8Args a) {
     using H = Half16<T>;
-    using P = typename H::pair;
     constexpr int MP = 8;
     constexpr uint32_t kItem = KB * 1024;
     extern __shared__ __align__(1024) uint8_t smem[];
@@ -123,61 +134,30 @@ int8_gemv_tma_kernel(const __grid_constant__ CUtensorMap wmap, const Tma8Args a)
     // ---- consumers ---------------------------------------------------------------------------
     const bool works = warp < active && t0 + warp / a.wpt < t1;
     const int ts = warp / a.wpt, part = warp % a.wpt;
-    const uint32_t xs = smem0 + lay.xs, xsum = smem0 + lay.xsum;
+    const uint32_t xs = smem0 + lay.xs;
 
     if (a.overlap) {
         if (a.early) pdl_launch_dependents();
         pdl_wait();  // activations may come from the kernel ahead of this one
     }
 
-    // Activations: M * (K / 8) pieces of 16 bytes (8 inputs), the 8 pieces of a (row, k-block) in
-    // 8 consecutive lanes, which also add up the k-block's inputs.
+    // Activations: M * (K / 8) pieces of 16 bytes, as they are.
     {
         const uint4* xg = below_pdl_wait(static_cast<const uint4*>(a.x));
-        const int pieces = M * kblocks * 8;
+        const int row_pieces = kblocks * 8, pieces = M * row_pieces;
         constexpr int threads = WARPS * 32;
-        const uint32_t sixteen_bits = H::pack(16.0f, 16.0f);
-        const P sixteen = *reinterpret_cast<const P*>(&sixteen_bits);
         for (int base = 0; base < pieces; base += 4 * threads) {  // four loads in flight a thread
             uint4 raw[4];
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
                 const int e = base + u * threads + int(threadIdx.x);
-                raw[u] = make_uint4(0, 0, 0, 0);
-                if (e < pieces) {
-                    const int r = e >> 3, c = e & 7;
-                    const int m = M == 1 ? 0 : r / kblocks, j = r - m * kblocks;
-                    raw[u] = ld_mutable(xg + (size_t(m) * K + size_t(j) * 64) / 8 + c);
-                }
+                if (e < pieces) raw[u] = ld_mutable(xg + e);
             }
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
                 const int e = base + u * threads + int(threadIdx.x);
-                const bool live = e < pieces;
-                const int r = e >> 3, c = e & 7;
-                const int m = M == 1 ? 0 : r / kblocks, j = r - m * kblocks;
-                float sum = (H::to_float(raw[u].x & 0xFFFFu) + H::to_float(raw[u].x >> 16)) +
-                            (H::to_float(raw[u].y & 0xFFFFu) + H::to_float(raw[u].y >> 16));
-                sum += (H::to_float(raw[u].z & 0xFFFFu) + H::to_float(raw[u].z >> 16)) +
-                       (H::to_float(raw[u].w & 0xFFFFu) + H::to_float(raw[u].w >> 16));
-#pragma unroll
-                for (int d = 4; d >= 1; d >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, d);
-                if (live && c == 0) sts32f(xsum + (uint32_t(m / 2) * kblocks + j) * 8 + (m % 2) * 4, sum);
-                if (live) {
-                    // piece c: inputs 8c .. 8c+7 of the k-block, the words i = 2 (c % 2) and + 1 of lane t = c / 2
-                    const uint32_t dst = xs + uint32_t(m) * lay.xrow + uint32_t(j) * 256 + (2 * (c & 1)) * 64 + (c >> 1) * 16;
-#pragma unroll
-                    for (int hh = 0; hh < 2; ++hh) {
-                        const uint32_t lo = hh == 0 ? raw[u].x : raw[u].z, hi = hh == 0 ? raw[u].y : raw[u].w;
-                        uint4 out;
-                        out.x = __byte_perm(lo, hi, 0x5410);  // (x0, x2)
-                        out.z = __byte_perm(lo, hi, 0x7632);  // (x1, x3)
-                        P p02 = __hmul2(*reinterpret_cast<P*>(&out.x), sixteen), p13 = __hmul2(*reinterpret_cast<P*>(&out.z), sixteen);
-                        out.y = *reinterpret_cast<uint32_t*>(&p02);
-                        out.w = *reinterpret_cast<uint32_t*>(&p13);
-                        sts128(dst + hh * 64, out);
-                    }
-                }
+                const int m = e >= row_pieces ? 1 : 0;  // one or two rows
+                if (e < pieces) sts128(xs + uint32_t(m) * lay.xrow + uint32_t(e - m * row_pieces) * 16, raw[u]);
             }
         }
     }
@@ -185,12 +165,10 @@ int8_gemv_tma_kernel(const __grid_constant__ CUtensorMap wmap, const Tma8Args a)
     if (!works) return;
 
     // ---- this warp's items --------------------------------------------------------------------
-    const uint32_t kMask = 0x000F000Fu;
-    const float kCorrection = 17.0f * H::kBias + 128.0f;  // what the magic and the +128 of the bytes add per unit of X
+    const float kUnit = H::kDtype == B200Q_BF16 ? 64.0f : 1.0f;  // what widen8 divides a weight by
     uint16_t* y = static_cast<uint16_t*>(a.y);
     const uint32_t wl = uint32_t(g) * 64 + t * 16;  // this lane's bytes of a k-block's row g
-    const uint32_t x_lane = xs + uint32_t(min(g, M - 1)) * lay.xrow + t * 16;
-    const uint32_t xsum_lane = xsum + uint32_t(min(t, lay.xpairs - 1)) * kblocks * 8;
+    const uint32_t x_lane = xs + uint32_t(min(g, M - 1)) * lay.xrow + t * 32;
     bool ok = true;
     int n = 0;
     int s = warp % S;
@@ -211,41 +189,24 @@ int8_gemv_tma_kernel(const __grid_constant__ CUtensorMap wmap, const Tma8Args a)
             __syncwarp();  // every lane has seen the phase
             if (lane == 0) bar_arrive(taken0 + warp * 8);
             const uint32_t wq = stage_addr + wl;
-            const uint32_t xq = x_lane + uint32_t(item) * (KB * 256);
-            const uint32_t xsq = xsum_lane + uint32_t(item) * (KB * 8);
+            const uint32_t xq = x_lane + uint32_t(item) * (KB * 128);
 #pragma unroll
             for (int j = 0; j < KB; ++j) {
                 const uint4 q0 = lds128(wq + j * 1024), q1 = lds128(wq + j * 1024 + 512);
-                float ka[4], kb[4];
+                const uint4 b0 = lds128(xq + j * 128), b1 = lds128(xq + j * 128 + 16);
+                const uint32_t w0[4] = {q0.x, q0.y, q0.z, q0.w}, w1[4] = {q1.x, q1.y, q1.z, q1.w};
+                const uint32_t b[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+                float k[2][4];  // two chains
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
-                    const uint4 b = lds128(xq + j * 256 + i * 64);
-                    const uint32_t w0 = (i == 0 ? q0.x : i == 1 ? q0.y : i == 2 ? q0.z : q0.w) ^ 0x80808080u;
-                    const uint32_t w1 = (i == 0 ? q1.x : i == 1 ? q1.y : i == 2 ? q1.z : q1.w) ^ 0x80808080u;
-                    uint32_t f0[4], f1[4];  // (l0, l2) (h0, h2) (l1, l3) (h1, h3) of rows g, g+8
-                    f0[0] = lop3_and_or(w0, kMask, H::kMagic);
-                    f0[1] = lop3_and_or(w0 >> 4, kMask, H::kMagic);
-                    f0[2] = lop3_and_or(w0 >> 8, kMask, H::kMagic);
-                    f0[3] = lop3_and_or(w0 >> 12, kMask, H::kMagic);
-                    f1[0] = lop3_and_or(w1, kMask, H::kMagic);
-                    f1[1] = lop3_and_or(w1 >> 4, kMask, H::kMagic);
-                    f1[2] = lop3_and_or(w1 >> 8, kMask, H::kMagic);
-                    f1[3] = lop3_and_or(w1 >> 12, kMask, H::kMagic);
-                    const uint32_t a_lo[4] = {f0[0], f1[0], f0[1], f1[1]};
-                    const uint32_t a_hi[4] = {f0[2], f1[2], f0[3], f1[3]};
-                    if (i == 0) {
-                        mma_first<T>(ka, a_lo, b.x, b.y);
-                        mma_first<T>(kb, a_hi, b.z, b.w);
-                    } else {
-                        H::mma(ka, a_lo, b.x, b.y);
-                        H::mma(kb, a_hi, b.z, b.w);
-                    }
+                    const uint32_t u0 = w0[i] ^ 0x80808080u, u1 = w1[i] ^ 0x80808080u;
+                    const uint32_t f[4] = {widen8(u0, false, T{}), widen8(u1, false, T{}),   // rows g, g + 8: first pair
+                                           widen8(u0, true, T{}), widen8(u1, true, T{})};    // second pair
+                    if (i < 2) mma_first<T>(k[i], f, b[2 * i], b[2 * i + 1]);
+                    else H::mma(k[i - 2], f, b[2 * i], b[2 * i + 1]);
                 }
-                const float2 X = lds64f(xsq + j * 8);
-                acc[0] += fmaf(-kCorrection, X.x, ka[0] + kb[0]);
-                acc[1] += fmaf(-kCorrection, X.y, ka[1] + kb[1]);
-                acc[2] += fmaf(-kCorrection, X.x, ka[2] + kb[2]);
-                acc[3] += fmaf(-kCorrection, X.y, ka[3] + kb[3]);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) acc[e] += k[0][e] + k[1][e];
             }
             if (o + 1 < a.opc) {  // hand the stage back; the tile's last one carries the partial sums first
                 __syncwarp();
@@ -277,7 +238,7 @@ int8_gemv_tma_kernel(const __grid_constant__ CUtensorMap wmap, const Tma8Args a)
                     sum += lds32f(smem0 + uint32_t(sw) * kItem + (row * MP + m) * 4);
                 }
                 const int nrow = tile * 16 + row;
-                if (nrow < N) y[size_t(m) * N + nrow] = H::from_float(sum * __ldg(a.scale + nrow));
+                if (nrow < N) y[size_t(m) * N + nrow] = H::from_float(sum * kUnit * __ldg(a.scale + nrow));
             }
             __syncwarp();
             if (lane < a.wpt) bar_arrive(empty0 + (s_mine + lane < S ? s_mine + lane : s_mine + lane - S) * 8);
