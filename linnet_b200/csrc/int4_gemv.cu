@@ -446,17 +446,17 @@ bool run_tma(const GemvArgs& a, cudaStream_t stream, int32_t* status, const Norm
               (a.flags & B200Q_NO_OVERLAP) ? 0 : 1, (a.flags & B200Q_EARLY_DEPENDENTS) ? 1 : 0, (a.flags & B200Q_SWIGLU_INPUT) ? 1 : 0,
               norm ? norm->delta : nullptr, norm ? norm->weight : nullptr, norm ? norm->x_out : nullptr,
               norm ? norm->eps : 0.0f, word};
-    size_t smem = 0;
     const int sms = sm_count();
-    if (tma_plan<1, 16, 8>(p, a.G, &smem)) {
-        *status = launch_tma<T, 1, 16, 8, false>(p, a.packed, smem, sms, stream);
+    TmaArgs half = p;  // items of half the size: twice the warps a tile
+    size_t smem = 0, half_smem = 0;
+    const bool whole = tma_plan<1, 16, 8>(p, a.G, &smem), halves = tma_plan<1, 16, 4>(half, a.G, &half_smem);
+    if (halves && (!whole || half_items_pay(half, sms))) {
+        *status = launch_tma<T, 1, 16, 4, false>(half, a.packed, half_smem, sms, stream);
         return true;
     }
-    if (tma_plan<1, 16, 4>(p, a.G, &smem)) {
-        *status = launch_tma<T, 1, 16, 4, false>(p, a.packed, smem, sms, stream);
-        return true;
-    }
-    return false;
+    if (!whole) return false;
+    *status = launch_tma<T, 1, 16, 8, false>(p, a.packed, smem, sms, stream);
+    return true;
 }
 
 template <typename T>

@@ -275,17 +275,17 @@ bool run_tma8(const Gemv8Args& a, cudaStream_t stream, int32_t* status) {
     if (word == nullptr) return false;
     Tma8Args p{a.x, a.scale, a.y, a.M, a.K, a.N, (a.N + 15) / 16, 1, 1, 1, 0, 1,
                (a.flags & B200Q_EARLY_DEPENDENTS) ? 1 : 0, word};
-    size_t smem = 0;
     const int sms = sm_count();
-    if (tma8_plan<16, 8>(p, &smem)) {
-        *status = launch_tma8<T, 16, 8>(p, a.w, smem, sms, stream);
+    Tma8Args half = p;  // items of half the size: twice the warps a tile
+    size_t smem = 0, half_smem = 0;
+    const bool whole = tma8_plan<16, 8>(p, &smem), halves = tma8_plan<16, 4>(half, &half_smem);
+    if (halves && (!whole || half_items_pay(half, sms) || half.producers > p.producers)) {
+        *status = launch_tma8<T, 16, 4>(half, a.w, half_smem, sms, stream);
         return true;
     }
-    if (tma8_plan<16, 4>(p, &smem)) {
-        *status = launch_tma8<T, 16, 4>(p, a.w, smem, sms, stream);
-        return true;
-    }
-    return false;
+    if (!whole) return false;
+    *status = launch_tma8<T, 16, 8>(p, a.w, smem, sms, stream);
+    return true;
 }
 
 // Up to this many rows the tensor-core product starts early, as the decode kernels do.

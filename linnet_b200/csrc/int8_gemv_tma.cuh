@@ -10,7 +10,7 @@
 // times 2^127 less 2 is (u - 128) / 64, exact in 8 bits; in f16 0x6400 | u is 1024 + u, less 1152 is
 // w.  Five instructions (three of the integer pipe) and one MMA a word of four weights.  Before, a
 // byte was taken as two 4-bit planes: seven integer instructions and two MMAs a word, and sums of
-// (128 + q) that a correction had to bring back; 18.0 us a launch at 4096 -> 14336 against 16.3 now,
+// (128 + q) that a correction had to bring back; 18.0 us a launch at 4096 -> 14336 against 16.3,
 // two rows at 14336 -> 4096 30.2 against 16.6.
 // The per-row scale multiplies the finished sum, as in the kernel this one
 // relieves for one and two rows (int8_gemv.cu), and as linnet::gemv8 does
@@ -28,6 +28,17 @@
 
 namespace b200q {
 
+// Producer threads (one a warp) of a block.  Sending an item (two barrier tests, the byte count, the
+// copy) takes one thread about 450 clocks, and the 16 consumers want one more often than that: one
+// -> four producers, us a launch: 4096 -> 14336 16.3 -> 13.8, 4096 -> 28672 28.8 -> 22.9 (5.1 TB/s),
+// 14336 -> 4096 16.0 -> 13.7, 4096 -> 6144 7.8 -> 6.9.  (The int4 kernel, whose consumers take
+// longer, got 2 to 5 % slower.)  Each producer has its own consumers and its own stages of the ring,
+// every `producers`-th of both: a producer that left out a lap of a barrier could not tell its phase
+// from the one after next, so their number divides the warps of a tile (and with them every round's
+// items) and the stages.
+constexpr int kProducers = 4;
+inline int tma_producers(int wpt) { return wpt % 4 == 0 ? 4 : wpt % 2 == 0 ? 2 : 1; }
+
 struct Tma8Args {
     const void* x;       // [M, K]
     const float* scale;  // [N]
@@ -41,6 +52,7 @@ struct Tma8Args {
     int overlap;         // launched with programmatic stream serialization
     int early;           // dependents may start as soon as this kernel has started
     int* status;         // device word of expired waits
+    int producers;       // threads that send items; wpt and stages are multiples of it
 };
 
 struct Tma8Layout {
@@ -72,7 +84,7 @@ __device__ __forceinline__ uint32_t widen8(uint32_t u, bool second, __nv_bfloat1
 }
 
 template <typename T, int WARPS, int KB>
-__global__ void __launch_bounds__((WARPS + 1) * 32, 1)
+__global__ void __launch_bounds__((WARPS + kProducers) * 32, 1)
 int8_gemv_tma_kernel(const __grid_constant__ CUtensorMap wmap, const Tma8Args a) {
     using H = Half16<T>;
     constexpr int MP = 8;
@@ -99,32 +111,31 @@ int8_gemv_tma_kernel(const __grid_constant__ CUtensorMap wmap, const Tma8Args a)
     }
     __syncthreads();
 
-    if (warp == WARPS) {
-        // ---- producer: items in the order (round, item of the tile, consumer) ----------------
-        if (lane != 0) return;
+    if (warp >= WARPS) {
+        // ---- producers: items in the order (round, item of the tile, consumer), every one of
+        // them a consumer's in `producers` and with it a stage's ------------------------------------
+        const int mine = warp - WARPS, producers = a.producers;
+        if (lane != 0 || mine >= producers) return;
         if (a.overlap) pdl_launch_dependents();  // this thread never waits on the previous kernel: weights are constants
-        int s = 0;
-        uint32_t lap = 0;
+        int s = mine;
+        uint32_t lap = 0;  // times the ring has been gone round
         bool ok = true;
-        int n = 0;
+        int n = 0;         // items each consumer has been sent
         for (int round = 0; round < rounds && ok; ++round) {
-            const int tiles_here = min(a.tpc, t1 - t0 - round * a.tpc);
+            const int tiles_here = min(a.tpc, t1 - t0 - round * a.tpc);  // the last round may be short
             for (int o = 0; o < a.opc && ok; ++o, ++n) {
-                int w = 0;
-                for (int ts = 0; ts < tiles_here && ok; ++ts) {
-                    const int tile = t0 + round * a.tpc + ts;
-                    for (int part = 0; part < a.wpt; ++part, ++w) {
-                        const uint32_t empty = empty0 + s * 8, ready = ready0 + w * 8;
-                        if (lap > 0) ok = bar_wait<true>(empty, (lap - 1) & 1, a.status, 21);
-                        if (ok && n > 0) ok = bar_wait<true>(taken0 + w * 8, (n - 1) & 1, a.status, 23);
-                        if (!ok) break;
-                        bar_expect(ready, kItem);
-                        tma_item(smem0 + uint32_t(s) * kItem, &wmap, tile * 16, (part * a.opc + o) * KB, ready);
-                        if (++s == S) {
-                            s = 0;
-                            ++lap;
-                        }
-                    }
+                int tile = t0 + round * a.tpc, part = mine;
+                for (int w = mine; w < tiles_here * a.wpt; w += producers) {
+                    const uint32_t empty = empty0 + s * 8, ready = ready0 + w * 8;
+                    if (lap > 0) ok = bar_wait<true>(empty, (lap - 1) & 1, a.status, 21);
+                    if (ok && n > 0) ok = bar_wait<true>(taken0 + w * 8, (n - 1) & 1, a.status, 23);
+                    if (!ok) break;
+                    bar_expect(ready, kItem);
+                    tma_item(smem0 + uint32_t(s) * kItem, &wmap, tile * 16, (part * a.opc + o) * KB, ready);
+                    s += producers;
+                    if (s >= S) s -= S, ++lap;
+                    part += producers;
+                    if (part >= a.wpt) part -= a.wpt, ++tile;
                 }
             }
         }
@@ -263,7 +274,9 @@ inline bool tma8_plan(Tma8Args& a, size_t* smem) {
     long stages = (budget - 2 * WARPS * 8 - 128) / (KB * 1024 + 8);
     if (stages < 4 || stages <= a.wpt) return false;
     if (stages > 96) stages = 96;
-    a.stages = int(stages);
+    a.producers = tma_producers(a.wpt);
+    if (stages / a.producers * a.producers <= a.wpt) a.producers = 1;
+    a.stages = int(stages) / a.producers * a.producers;
     *smem = tma8_layout<WARPS, KB>(a.M, a.K, a.stages).total;
     return true;
 }
@@ -295,7 +308,7 @@ int32_t launch_tma8(const Tma8Args& a, const int8_t* w, size_t smem, int sms, cu
     const int grid = a.tiles < sms ? a.tiles : sms;
     cudaLaunchConfig_t config = {};
     config.gridDim = dim3(unsigned(grid), 1, 1);
-    config.blockDim = dim3((WARPS + 1) * 32, 1, 1);
+    config.blockDim = dim3((WARPS + kProducers) * 32, 1, 1);
     config.dynamicSmemBytes = smem;
     config.stream = stream;
     cudaLaunchAttribute attr[1];

@@ -131,4 +131,17 @@ __device__ __forceinline__ void bar_expect(uint32_t bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
 
+// The decode kernels with a ring of weights cut a tile's K into items, one at a time a warp.  With
+// items of half the size twice as many warps share a tile, which pays while a block has work for at
+// most half of its 16 warps: int4, us a launch with whole -> half items: 1024 -> 1024 2.97 -> 2.45,
+// 1024 -> 4096 3.40 -> 2.89, 2048 -> 2048 3.21 -> 2.77, 2048 -> 4096 3.47 -> 3.39, but 4096 -> 4096
+// (16 half items) 4.69 -> 5.18 and 4096 -> 28672 16.9 -> 25.7: an item costs its producer thread as
+// much whatever its size.
+template <typename Args>
+inline bool half_items_pay(const Args& half, int sms) {
+    const int grid = half.tiles < sms ? half.tiles : sms;
+    const int most = (half.tiles + grid - 1) / grid;  // tiles of the busiest block
+    return most * half.wpt * half.opc <= 8;
+}
+
 }  // namespace b200q
