@@ -109,7 +109,8 @@ int32_t b200q_int4_gemv(const void* x, const uint8_t* packed, const void* scale,
  *     SwiGLU of a decoder layer without a launch of its own.  Taken for one or two rows,
  *     groups of 128 and the default numerics; B200Q_UNAVAILABLE otherwise (the caller then
  *     forms the input itself).  No counterpart in the reference.
- *   B200Q_NO_OVERLAP   the one- and two-row kernel is launched in plain stream order: it starts
+ *   B200Q_NO_OVERLAP   the one- and two-row kernel (and the tensor-core product, up to 64 rows) is
+ *     launched in plain stream order: it starts
  *     when everything before it in the stream has finished, instead of starting early and
  *     fetching weights while the kernel before it still runs (programmatic dependent launch,
  *     the default).  For callers that want plain stream order, and for timing the kernel
@@ -124,10 +125,10 @@ int32_t b200q_int4_linear_ex(const void* x, const uint8_t* packed, const void* s
                              int64_t out, int64_t group, int32_t dtype, int32_t flags,
                              void* stream);
 
-/* The prefill kernel alone: TMA + tcgen05/TMEM dequant-GEMM (bf16; `in` a multiple of 64,
+/* The tensor-core product alone: weights dequantized into tensor memory (bf16; `in` a multiple of 64,
  * `group` 64 times a power of two, a packed weight under 4 GB; any rows and out;
- * B200Q_ERROR otherwise: b200q_int4_linear sends such shapes to the decode kernels in
- * passes). */
+ * B200Q_ERROR otherwise).  b200q_int4_linear runs the same kernel for f16 and for groups of 16, 32
+ * and any multiple of 64 too, and sends other shapes to the decode kernels in passes. */
 int32_t b200q_int4_gemm(const void* x, const uint8_t* packed, const void* scale,
                         const uint8_t* zero, void* y, int64_t rows, int64_t in,
                         int64_t out, int64_t group, int32_t dtype, void* stream);
@@ -164,8 +165,9 @@ int32_t b200q_int4_dequantize(const uint8_t* packed, const void* scale,
  * y[rows, out] = x[rows, in] . (w * scale)^T, f32 accumulate.
  *   w [out, in] i8; scale f32: [out] when group == 0, else [out, in/group].
  * Replaces linnet::gemv8 (kernels.py:336-434, one row) and linnet::w8a16
- * (kernels.py:437-592, 2..64 rows) for the int8 formats; more rows run the same
- * tiles in passes until the tcgen05 path covers them. */
+ * (kernels.py:437-592, 2..64 rows) for the int8 formats.  From a few rows on the
+ * tensor-core product takes any row count (`in` a multiple of 64, one scale a row or groups of 16,
+ * 32 or a multiple of 64); other shapes run the decode kernel in passes of 16 rows. */
 int32_t b200q_int8_linear(const void* x, const int8_t* w, const float* scale,
                           void* y, int64_t rows, int64_t in, int64_t out,
                           int64_t group, int32_t dtype, void* stream);

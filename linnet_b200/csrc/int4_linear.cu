@@ -16,6 +16,7 @@ static constexpr int64_t kOverlapRows = 64;
 //     4096 -> 4096              4.8/10.6  11.4/10.6  11.8/10.7  18.2/11.9
 //     4096 -> 28672            23.4/31.2  30.5/31.3  31.4/31.3  59.3/31.2
 //     14336 -> 4096            13.6/19.7  26.2/19.7  26.6/19.8  50.9/21.0
+//     4096 -> 14336           12.5/17.3  15.2/17.4  15.9/17.4  30.0/17.9
 //   other groups                  1 row     3 rows     8 rows    16 rows
 //     32, 2048 -> 2048          5.1/7.4   5.4/7.4    6.4/7.5    8.2/7.5
 //     32, 4096 -> 4096        12.2/10.6 13.7/11.1  17.7/11.2  22.4/11.3
@@ -24,11 +25,19 @@ static constexpr int64_t kOverlapRows = 64;
 //     64, 4096 -> 14336       22.2/17.5 27.0/17.5  35.8/17.6  56.5/17.7
 //     256, 4096 -> 4096         6.1/9.8  7.5/10.3  13.9/10.6  18.6/10.6
 //     256, 4096 -> 14336      15.0/17.3 19.7/17.3  30.3/17.3  49.4/17.4
-static int64_t gemm_rows(int64_t weights, int64_t group) {
+// Over 150 drawn shapes one or two rows with other groups came out either way (0.75 to 1.5 times),
+// and 9 to 16 rows with groups of 128 lost up to a third where the product's tiles of 128 columns
+// leave its last round mostly empty and K is not split (9557 columns: 75 tiles on 148
+// multiprocessors, 26.4/38.8; 11468: 90 tiles, 26.3/33.0): those stay with the decode kernels.
+static int64_t gemm_rows(int64_t in, int64_t out, int64_t group) {
     constexpr int64_t kSome = int64_t(12) << 20, kMany = int64_t(32) << 20;  // weights: 3072 x 4096, 8192 x 4096
-    if (group == 128 || weights < kSome) return 9;
-    if (group < 64) return 1;
-    if (group == 64) return weights < kMany ? 3 : 1;
+    const int64_t weights = in * out;
+    if (group == 128) {
+        const int64_t tiles = (out + 127) / 128, sms = sm_count(), rounds = (tiles + sms - 1) / sms;
+        return tiles > sms / 2 && tiles * 10 < rounds * sms * 7 ? 17 : 9;
+    }
+    if (weights < kSome) return 9;
+    if (group <= 64) return weights < kMany ? 4 : 3;
     return weights < kMany ? 7 : 3;
 }
 
@@ -36,7 +45,7 @@ extern "C" int32_t b200q_int4_linear_ex(const void* x, const uint8_t* packed, co
                                         const uint8_t* zero, void* y, int64_t rows, int64_t in,
                                         int64_t out, int64_t group, int32_t dtype, int32_t flags,
                                         void* stream) {
-    if (rows >= gemm_rows(in * out, group) && !(flags & B200Q_SWIGLU_INPUT)) {
+    if (rows >= gemm_rows(in, out, group) && !(flags & B200Q_SWIGLU_INPUT)) {
         const int32_t ok = check_int4_args("int4_linear", x, packed, scale, zero, y, rows, in, out, group, dtype);
         if (ok != B200Q_OK) return ok;
         const WqProblem p{kWqInt4, x, packed, scale, zero, y, rows, in, out, group, dtype};

@@ -292,22 +292,22 @@ bool run_tma8(const Gemv8Args& a, cudaStream_t stream, int32_t* status) {
 constexpr int64_t kOverlapRows8 = 64;
 
 // Rows from which the tensor-core product is used (the same time from 1 to 64 rows; one or two rows
-// with one scale a row stay with int8_gemv_tma.cuh's kernel, whose sums take the scale unrounded).
+// stay with the decode kernels: those with one scale a row with int8_gemv_tma.cuh's, whose sums take
+// the scale unrounded, those with group scales came out 0.86 to 1.25 times over drawn shapes).
 // Decode kernel / tensor-core product, us a launch in a chain on a B200:
 //                                 1 row     3 rows     6 rows     8 rows    16 rows
 //   2048 -> 2048                5.2/7.9    5.6/7.9    5.9/8.0    6.0/8.0    8.3/8.0
 //   4096 -> 4096               9.4/10.5   9.9/10.7  10.4/11.0  15.7/11.0  12.3/11.0
 //   4096 -> 14336             22.0/18.0  23.7/17.9  31.4/17.9  32.5/17.9  40.7/18.0
 //   14336 -> 4096             24.8/19.5  34.2/19.9  35.5/20.2  36.9/20.2  45.2/20.2
-int64_t gemm_rows8(int64_t weights, bool one_scale_a_row) {
+int64_t gemm_rows8(int64_t weights) {
     if (weights < (int64_t(12) << 20)) return 9;   // 3072 x 4096
-    if (weights < (int64_t(32) << 20)) return 7;   // 8192 x 4096
-    return one_scale_a_row ? 3 : 1;
+    return weights < (int64_t(32) << 20) ? 7 : 3;  // 8192 x 4096
 }
 
 template <typename T>
 int32_t run_gemv8(Gemv8Args a, int64_t rows, cudaStream_t stream) {
-    if (rows >= gemm_rows8(int64_t(a.K) * a.N, a.G == 0 || a.G == a.K)) {
+    if (rows >= gemm_rows8(int64_t(a.K) * a.N)) {
         // the same weights as the decode kernel's below: scaled in f32, rounded once
         const WqProblem p{kWqInt8, a.x, a.w, a.scale, nullptr, a.y, rows, a.K, a.N, a.G == 0 ? a.K : a.G, Half16<T>::kDtype};
         if (wq_gemm_supports(p)) return wq_gemm("int8_linear", p, rows <= kOverlapRows8, stream);

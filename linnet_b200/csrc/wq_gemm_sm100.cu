@@ -18,16 +18,25 @@
 //
 // One persistent block per multiprocessor, 24 warps with fixed roles:
 //   warps 0-3   epilogue: tensor memory -> registers -> 16-bit -> Y
-//   warp  4, 5  TMA producers of X (64 inputs x nx rows a stage) and W (128 inputs x 128 rows)
-//   warp  6     issues tcgen05.mma;  warp 7 allocates tensor memory
+//   warp  4, 5  TMA producers of X (128 inputs x nx rows a stage) and W (128 inputs x 128 rows)
+//   warp  6, 7  issue tcgen05.mma (7 also allocates tensor memory)
 //   warps 8-23  dequantizers: four teams of four warps (a warp may touch the 32 lanes of its
-//               quarter only), taking the ITEMS of 64 inputs x 128 rows in turn
+//               quarter only); two teams share an ITEM of 128 inputs x 128 rows, half the inputs each
 // A block tile is R * 128 rows of W (R accumulators fed by the same activations: wide tiles halve
 // the traffic of X that way) by nx rows of X.  Where the tiles would leave multiprocessors idle a
 // cluster of k_splits blocks shares a tile, each a slice of K; their f32 sums meet in distributed
 // shared memory, in the order of the slices.  No global scratch, no atomics on results.
 // Every wait on an mbarrier is bounded: on expiry the block raises an error flag in global memory,
-// stops issuing work, still releases its tensor memory and returns.
+// stops issuing work, waits for its copies in flight, still releases its tensor memory and returns.
+//
+// What bounds it: the dequantizers' integer pipe for few rows (about 700 clocks an item, 28 weights a
+// clock and multiprocessor), the tensor pipe and the chip's power for prompts.  In a chain of launches
+// on a B200, us, against the kernels this one took over from (decode kernels in passes, a bf16-only
+// tensor-core kernel with dequantized weights in shared memory):
+//   int4 g128 bf16    16 x 14336 -> 4096   26.6 -> 18.4     128 x 4096 -> 28672   58 -> 34
+//                   2048 x 4096 -> 28672  392 -> 375..400 (power)
+//   int4 g32           16 x 4096 -> 28672 109.7 -> 30.5
+//   int8               64 x 4096 -> 14336 154.8 -> 20.5     200 x 4096 -> 14336  508.6 -> 29.8
 #include <atomic>
 
 #include "mma.cuh"
@@ -735,11 +744,11 @@ int resident_clusters(int splits) {
 // An item (128 inputs x 128 rows of W) takes the products kProductClocks a column (kWideX times
 // that where one block of rows is fed from wide tiles of X: shared memory), the dequantizers
 // kItemClocks and one issuing warp kIssueClocks; a tile that cannot double-buffer its accumulators
-// pays for its epilogue, a K split for the exchange.  The constants are fitted to 1,000 measured
-// launches (16 to 2048 rows on five weights, every tile shape); the shapes they choose are within
-// 1.1 % of the best measured ones on average, 15 % at worst.
-constexpr double kItemClocks = 694, kIssueClocks = 1042, kTileClocks = 1113, kSplitClocks = 14600, kColumnClocks = 69,
-                 kProductClocks = 2.82, kWideX = 1.83;
+// pays kColumnClocks a column for its epilogue, a K split kSplitClocks and kExchangeClocks a column.
+// The constants are fitted to 1,000 measured launches (16 to 2048 rows on five weights, every tile
+// shape); the shapes they choose are within 1.6 % of the best measured ones on average.
+constexpr double kItemClocks = 766, kIssueClocks = 1031, kTileClocks = 1200, kSplitClocks = 3200, kExchangeClocks = 78,
+                 kColumnClocks = 48, kProductClocks = 3.5, kWideX = 1.58;
 
 bool choose_plan(const WqProblem& q, WqPlan* best) {
     const int chunks = int((q.in + kChunk - 1) / kChunk);
@@ -764,7 +773,7 @@ bool choose_plan(const WqProblem& q, WqPlan* best) {
                 if (item < kItemClocks) item = kItemClocks;
                 if (issuers == 1 && item < kIssueClocks) item = kIssueClocks;
                 const double epilogue = kColumnClocks * R * nx;
-                const double tile = double((chunks + splits - 1) / splits) * R * item + (splits > 1 ? kSplitClocks : 0) +
+                const double tile = double((chunks + splits - 1) / splits) * R * item + (splits > 1 ? kSplitClocks + kExchangeClocks * nx : 0) +
                                     kTileClocks + (p.acc_bufs == 1 ? epilogue : 0);
                 const double cost = double((tiles + slots - 1) / slots) * tile + (p.acc_bufs == 2 ? epilogue : 0);
                 if (!found || cost < best_cost) *best = p, best_cost = cost, found = true;
@@ -872,9 +881,10 @@ extern "C" int32_t b200q_int4_gemm(const void* x, const uint8_t* packed, const v
     if (ok != B200Q_OK || rows == 0) return ok;
     const WqProblem p{kWqInt4, x, packed, scale, zero, y, rows, in, out, group, dtype};
     const int64_t items = group / kStep;
-    B200Q_REQUIRE(dtype == B200Q_BF16 && group % kStep == 0 && (items & (items - 1)) == 0 && wq_gemm_supports(p),
-                  "int4_gemm: needs bf16, inputs a multiple of %d, a group of that many times a power of two (got in=%lld "
-                  "group=%lld)", kStep, (long long)in, (long long)group);
+    B200Q_REQUIRE(dtype == B200Q_BF16 && group % kStep == 0 && (items & (items - 1)) == 0 &&
+                      out * (in / 2) < (int64_t(1) << 32) && wq_gemm_supports(p),
+                  "int4_gemm: needs bf16, inputs a multiple of %d, a group of that many times a power of two, a packed "
+                  "weight under 4 GB (got in=%lld group=%lld)", kStep, (long long)in, (long long)group);
     return wq_gemm("int4_gemm", p, false, static_cast<cudaStream_t>(stream));
 }
 
