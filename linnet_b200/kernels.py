@@ -106,7 +106,10 @@ def _int4_linear(x: torch.Tensor, packed: torch.Tensor, scale: torch.Tensor,
     if packed.dtype != torch.uint8 or zero.dtype != torch.uint8:
         raise ValueError("int4_linear: packed weights and zero points are uint8")
     device = _on_gpu("int4_linear", x, packed, scale, zero)
+    weight = (packed, scale, zero)
     x, packed, scale, zero = x.contiguous(), packed.contiguous(), scale.contiguous(), zero.contiguous()
+    if packed is not weight[0] or scale is not weight[1] or zero is not weight[2]:
+        overlap = False  # copied just now: no fetch of the weights ahead of the kernel that writes them
     if out is None:
         y = torch.empty(rows, width, dtype=x.dtype, device=device)
     else:
@@ -277,7 +280,8 @@ def gemv8(x: torch.Tensor, weight: torch.Tensor, scale: torch.Tensor, fp8: bool,
 
 def w8a16(x: torch.Tensor, weight: torch.Tensor, scale: torch.Tensor, fp8: bool, group: int,
           row_block: int) -> torch.Tensor:
-    """`F.linear(x, W)` for a few rows `x` [rows, In]; same weights as `gemv8`."""
+    """`F.linear(x, W)` for rows `x` [rows, In]; same weights as `gemv8`.  Any row count where
+    `w8a16_any_rows` says so, else a few."""
     if torch.compiler.is_compiling():
         return _w8a16_op(x, weight, scale, fp8, group, row_block)
     return _eight_bit("w8a16", x, weight, scale, fp8, group, row_block)
