@@ -301,6 +301,7 @@ constexpr int64_t kOverlapRows8 = 64;
 //   4096 -> 14336             22.0/18.0  23.7/17.9  31.4/17.9  32.5/17.9  40.7/18.0
 //   14336 -> 4096             24.8/19.5  34.2/19.9  35.5/20.2  36.9/20.2  45.2/20.2
 int64_t gemm_rows8(int64_t weights) {
+    if (weights < (int64_t(6) << 20)) return 14;   // 1536 x 4096 (2048 x 1536, 13 rows: 6.5/7.2)
     if (weights < (int64_t(12) << 20)) return 9;   // 3072 x 4096
     return weights < (int64_t(32) << 20) ? 7 : 3;  // 8192 x 4096
 }
