@@ -49,9 +49,10 @@ extern "C" int32_t b200q_int4_linear_ex(const void* x, const uint8_t* packed, co
         const int32_t ok = check_int4_args("int4_linear", x, packed, scale, zero, y, rows, in, out, group, dtype);
         if (ok != B200Q_OK) return ok;
         const WqProblem p{kWqInt4, x, packed, scale, zero, y, rows, in, out, group, dtype};
-        if (wq_gemm_supports(p))
-            return wq_gemm("int4_linear", p, rows <= kOverlapRows && !(flags & B200Q_NO_OVERLAP),
-                           static_cast<cudaStream_t>(stream));
+        const WqStart start = (flags & B200Q_NO_OVERLAP) ? WqStart::kStreamOrder
+                              : rows <= kOverlapRows     ? WqStart::kFetchAhead
+                                                         : WqStart::kEarly;
+        if (wq_gemm_supports(p)) return wq_gemm("int4_linear", p, start, static_cast<cudaStream_t>(stream));
     }
     return b200q_int4_gemv_ex(x, packed, scale, zero, y, rows, in, out, group, dtype, flags, stream);
 }

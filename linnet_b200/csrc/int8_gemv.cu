@@ -33,7 +33,7 @@ struct Gemv8Args {
     int kblocks;         // K / 64
     int kb_per_cta;
     int ksplit;
-    int flags;           // B200Q_EXACT_WEIGHTS | B200Q_EARLY_DEPENDENTS
+    int flags;           // B200Q_EXACT_WEIGHTS | B200Q_EARLY_DEPENDENTS | B200Q_NO_OVERLAP
 };
 
 template <int NT>
@@ -248,7 +248,7 @@ int32_t launch_gemv8(const Gemv8Args& args, int ksplit, cudaStream_t stream) {
     const int tiles = (a.N + 16 * NT - 1) / (16 * NT);
     const size_t smem = size_t(a.kb_per_cta) * 8 * a.M * 16 + size_t(W) * NT * 16 * MB * 8 * 4;
     return launch_clustered("int8_gemv", int8_gemv_kernel<T, MODE, MB, NT, W, D>, a, tiles, ksplit,
-                            W * 32, smem, stream, true);
+                            W * 32, smem, stream, !(a.flags & B200Q_NO_OVERLAP));
 }
 
 template <typename T, int MODE>
@@ -273,7 +273,7 @@ bool run_tma8(const Gemv8Args& a, cudaStream_t stream, int32_t* status) {
     if (size_t(a.N) * size_t(a.K) >= (size_t(1) << 40)) return false;
     int* word = gemm_error_word();
     if (word == nullptr) return false;
-    Tma8Args p{a.x, a.scale, a.y, a.M, a.K, a.N, (a.N + 15) / 16, 1, 1, 1, 0, 1,
+    Tma8Args p{a.x, a.scale, a.y, a.M, a.K, a.N, (a.N + 15) / 16, 1, 1, 1, 0, (a.flags & B200Q_NO_OVERLAP) ? 0 : 1,
                (a.flags & B200Q_EARLY_DEPENDENTS) ? 1 : 0, word};
     const int sms = sm_count();
     Tma8Args half = p;  // items of half the size: twice the warps a tile
@@ -311,7 +311,10 @@ int32_t run_gemv8(Gemv8Args a, int64_t rows, cudaStream_t stream) {
     if (rows >= gemm_rows8(int64_t(a.K) * a.N)) {
         // the same weights as the decode kernel's below: scaled in f32, rounded once
         const WqProblem p{kWqInt8, a.x, a.w, a.scale, nullptr, a.y, rows, a.K, a.N, a.G == 0 ? a.K : a.G, Half16<T>::kDtype};
-        if (wq_gemm_supports(p)) return wq_gemm("int8_linear", p, rows <= kOverlapRows8, stream);
+        const WqStart start = (a.flags & B200Q_NO_OVERLAP) ? WqStart::kStreamOrder
+                              : rows <= kOverlapRows8      ? WqStart::kFetchAhead
+                                                           : WqStart::kEarly;
+        if (wq_gemm_supports(p)) return wq_gemm("int8_linear", p, start, stream);
     }
     const uint8_t* x = static_cast<const uint8_t*>(a.x);
     uint8_t* y = static_cast<uint8_t*>(a.y);
@@ -348,7 +351,8 @@ using namespace b200q;
 extern "C" int32_t b200q_int8_linear_ex(const void* x, const int8_t* w, const float* scale, void* y,
                                         int64_t rows, int64_t in, int64_t out, int64_t group,
                                         int32_t dtype, int32_t flags, void* stream) {
-    B200Q_REQUIRE((flags & ~(B200Q_EXACT_WEIGHTS | B200Q_EARLY_DEPENDENTS)) == 0, "int8_linear: unknown flag bits %d", flags);
+    B200Q_REQUIRE((flags & ~(B200Q_EXACT_WEIGHTS | B200Q_EARLY_DEPENDENTS | B200Q_NO_OVERLAP)) == 0,
+                  "int8_linear: unknown flag bits %d", flags);
     B200Q_REQUIRE(dtype == B200Q_BF16 || dtype == B200Q_F16, "int8_linear: activations are bf16 or f16");
     B200Q_REQUIRE(rows >= 0 && in > 0 && out > 0, "int8_linear: bad shape rows=%lld in=%lld out=%lld",
                   (long long)rows, (long long)in, (long long)out);

@@ -21,7 +21,12 @@ struct WqProblem {
 
 // Whether the kernel takes this problem (at least one row; pointers as the entry points check them).
 bool wq_gemm_supports(const WqProblem& p);
-// Launches it; `overlap`: with programmatic stream serialization.
-int32_t wq_gemm(const char* who, const WqProblem& p, bool overlap, cudaStream_t stream);
+// What the launch may do while the kernels before it in the stream still run.
+enum class WqStart {
+    kStreamOrder,  // nothing: an ordinary launch
+    kEarly,        // start, set up its barriers and tensor memory, then wait for them
+    kFetchAhead,   // fetch and convert weights too: nothing in flight may be writing those
+};
+int32_t wq_gemm(const char* who, const WqProblem& p, WqStart start, cudaStream_t stream);
 
 }  // namespace b200q

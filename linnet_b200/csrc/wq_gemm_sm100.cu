@@ -795,7 +795,7 @@ bool wq_gemm_supports(const WqProblem& p) {
     return aligned(p.scale, size_t(4 * gps));
 }
 
-int32_t wq_gemm(const char* who, const WqProblem& q, bool overlap, cudaStream_t stream) {
+int32_t wq_gemm(const char* who, const WqProblem& q, WqStart start, cudaStream_t stream) {
     EncodeTiled encode = encode_tiled();
     if (encode == nullptr) return unavailable("%s: the driver has no cuTensorMapEncodeTiled", who);
     WqPlan p;
@@ -831,7 +831,7 @@ int32_t wq_gemm(const char* who, const WqProblem& q, bool overlap, cudaStream_t 
     a.x_stages = p.x_stages, a.w_stages = p.w_stages, a.slots = p.slots, a.acc_bufs = p.acc_bufs;
     a.w_ring = uint32_t(p.w_ring), a.exchange = uint32_t(p.exchange), a.barriers = uint32_t(p.barriers);
     a.pairs = q.out % 2 == 0 && aligned(q.y, 4);
-    a.wait_weights = !overlap;
+    a.wait_weights = start != WqStart::kFetchAhead;
 
     const WqKernel kernel = q.dtype == B200Q_BF16 ? pick<__nv_bfloat16>(q.format, q.group) : pick<__half>(q.format, q.group);
     const cudaError_t limit = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), p.smem);
@@ -843,13 +843,19 @@ int32_t wq_gemm(const char* who, const WqProblem& q, bool overlap, cudaStream_t 
     config.dynamicSmemBytes = p.smem;
     config.stream = stream;
     cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    attr[1].id = cudaLaunchAttributeClusterDimension;
-    attr[1].val.clusterDim.x = unsigned(p.splits);
-    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+    unsigned attrs = 0;
+    if (start != WqStart::kStreamOrder) {
+        attr[attrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[attrs++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (p.splits > 1) {
+        attr[attrs].id = cudaLaunchAttributeClusterDimension;
+        attr[attrs].val.clusterDim.x = unsigned(p.splits);
+        attr[attrs].val.clusterDim.y = attr[attrs].val.clusterDim.z = 1;
+        ++attrs;
+    }
     config.attrs = attr;
-    config.numAttrs = p.splits > 1 ? 2 : 1;
+    config.numAttrs = attrs;
     return launch_status(who, cudaLaunchKernelEx(&config, kernel, x_map, w_map, a));
 }
 
@@ -885,7 +891,7 @@ extern "C" int32_t b200q_int4_gemm(const void* x, const uint8_t* packed, const v
                       out * (in / 2) < (int64_t(1) << 32) && wq_gemm_supports(p),
                   "int4_gemm: needs bf16, inputs a multiple of %d, a group of that many times a power of two, a packed "
                   "weight under 4 GB (got in=%lld group=%lld)", kStep, (long long)in, (long long)group);
-    return wq_gemm("int4_gemm", p, false, static_cast<cudaStream_t>(stream));
+    return wq_gemm("int4_gemm", p, WqStart::kEarly, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int32_t b200q_int4_gemm_status(void) {

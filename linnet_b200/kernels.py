@@ -237,13 +237,17 @@ def _eight_bit(who: str, x: torch.Tensor, weight: torch.Tensor, scale: torch.Ten
     if weight.shape[1] != depth:
         raise ValueError(f"{who}: x has {depth} inputs, the weight {weight.shape[1]}")
     device = _on_gpu(who, x, weight, scale)
+    given = (weight, scale)
     x, weight = x.contiguous(), weight.contiguous()
     scale = scale.float().contiguous()
+    # copied just now: no fetch of them ahead of the kernel that writes them
+    copied = weight is not given[0] or scale is not given[1]
+    flags = (_lib.EXACT_WEIGHTS if _exact_weights else 0) | (_lib.NO_OVERLAP if copied else 0)
     y = torch.empty(rows, width, dtype=x.dtype, device=device)
     with _Device(device):
         _lib.check(_lib.load().b200q_int8_linear_ex(
             x.data_ptr(), weight.data_ptr(), scale.data_ptr(), y.data_ptr(), rows, depth, width,
-            group, _code(x.dtype, who), _lib.EXACT_WEIGHTS if _exact_weights else 0, _stream(device)))
+            group, _code(x.dtype, who), flags, _stream(device)))
     return y
 
 
