@@ -109,13 +109,12 @@ int32_t b200q_int4_gemv(const void* x, const uint8_t* packed, const void* scale,
  *     SwiGLU of a decoder layer without a launch of its own.  Taken for one or two rows,
  *     groups of 128 and the default numerics; B200Q_UNAVAILABLE otherwise (the caller then
  *     forms the input itself).  No counterpart in the reference.
- *   B200Q_NO_OVERLAP   the one- and two-row kernel and the tensor-core product are
- *     launched in plain stream order: they start
- *     when everything before them in the stream has finished, instead of starting early and
- *     (the product up to 64 rows) fetching weights, scales and zero points while the kernel before
- *     still runs (programmatic dependent launch, the default).  For callers whose weights a kernel
- *     still in flight may be writing, and for timing the kernel
- *     without a neighbour's overlap.  No counterpart in the reference. */
+ *   B200Q_NO_OVERLAP   the kernel is launched in plain stream order: it starts when everything
+ *     before it in the stream has finished, instead of starting early and (the tensor-core product:
+ *     up to 64 rows) fetching weights, scales and zero points while the kernel before it still runs
+ *     (programmatic dependent launch, the default).  For callers whose weights a kernel still in
+ *     flight may be writing, and for timing the kernel without a neighbour's overlap.  No
+ *     counterpart in the reference. */
 enum { B200Q_EXACT_WEIGHTS = 1, B200Q_EARLY_DEPENDENTS = 2, B200Q_SWIGLU_INPUT = 4, B200Q_NO_OVERLAP = 8 };
 int32_t b200q_int4_gemv_ex(const void* x, const uint8_t* packed, const void* scale,
                            const uint8_t* zero, void* y, int64_t rows, int64_t in,
@@ -182,8 +181,7 @@ int32_t b200q_int8_linear(const void* x, const int8_t* w, const float* scale,
  *     the TMA unit, and a bounded wait of it that expires is reported by
  *     b200q_int4_gemm_status().
  *   B200Q_EARLY_DEPENDENTS   as for b200q_int4_gemv_ex.
- *   B200Q_NO_OVERLAP   every kernel of this entry is launched in plain stream order: weights and
- *     scales may come from the kernel before.  Without it they are fetched early. */
+ *   B200Q_NO_OVERLAP   as for b200q_int4_gemv_ex. */
 int32_t b200q_int8_linear_ex(const void* x, const int8_t* w, const float* scale,
                              void* y, int64_t rows, int64_t in, int64_t out,
                              int64_t group, int32_t dtype, int32_t flags, void* stream);

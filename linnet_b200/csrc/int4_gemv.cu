@@ -306,7 +306,7 @@ int32_t launch_gemv(const GemvArgs& args, int ksplit, cudaStream_t stream) {
     const size_t cap = (a.kb_per_cta + W - 1) / W;  // k-blocks per warp, at most
     const size_t smem = size_t(W) * cap * 16 * a.M * 16 + size_t(W) * NT * 16 * MB * 8 * 4;
     return launch_clustered("int4_gemv", int4_gemv_kernel<T, MODE, MB, NT, W, D>, a, tiles, ksplit,
-                            W * 32, smem, stream, true);
+                            W * 32, smem, stream, !(a.flags & B200Q_NO_OVERLAP));
 }
 
 template <typename T, int MODE>
@@ -326,7 +326,8 @@ bool run_rows(const GemvArgs& a, cudaStream_t stream, int32_t* status) {
     for (int c = 1; c <= octs; ++c)
         if (octs % c == 0 && octs / c <= 8) { opc = c; break; }
     if (opc == 0) return false;
-    RowsArgs r{a.x, a.packed, a.scale, a.zero, a.y, a.M, a.K, a.N, (a.N + 15) / 16, opc, octs / opc};
+    RowsArgs r{a.x, a.packed, a.scale, a.zero, a.y, a.M, a.K, a.N, (a.N + 15) / 16, opc, octs / opc,
+               (a.flags & B200Q_NO_OVERLAP) ? 0 : 1};
     const int sms = sm_count();
     // Widest block (most sharing of the staged activations) among those that keep every
     // block resident at once and still put a block on every multiprocessor.
@@ -381,9 +382,9 @@ bool run_short(OctArgs o, int G, cudaStream_t stream, int32_t* status) {
 // (of 4, 7, 2, 1) that divide K / 1024 with at most 8 blocks per cluster.
 template <typename T>
 bool run_oct(const GemvArgs& a, cudaStream_t stream, int32_t* status) {
-    // Every variant is launched with programmatic stream serialization: its weight
-    // prefetch overlaps the tail of the kernel before it.
-    OctArgs o{a.x, a.packed, a.scale, a.zero, a.y, a.M, a.K, a.N, 1, 1,
+    // Every variant is launched with programmatic stream serialization unless the caller asks
+    // for plain stream order: its weight prefetch overlaps the tail of the kernel before it.
+    OctArgs o{a.x, a.packed, a.scale, a.zero, a.y, a.M, a.K, a.N, 1, (a.flags & B200Q_NO_OVERLAP) ? 0 : 1,
               (a.flags & B200Q_EARLY_DEPENDENTS) ? 1 : 0};
     const bool few = a.M <= 8;
     if (few && a.G == 128) {

@@ -29,6 +29,7 @@ struct RowsArgs {
     int tiles;              // ceil(N / 16)
     int opc;                // octs per block
     int ksplit;             // blocks per cluster = K / (1024 * opc)
+    int overlap;            // launched with programmatic stream serialization
 };
 
 template <typename T, int MB, int W, int D>
@@ -225,7 +226,7 @@ int32_t launch_rows(RowsArgs a, cudaStream_t stream) {
     const size_t smem = size_t(8) * 4 * (MB * 8) * 4 * 16 + size_t(W) * 16 * (MB * 8) * 4;
     const int blocks = (a.tiles + W - 1) / W;
     return launch_clustered("int4_gemv", int4_gemv_rows_kernel<T, MB, W, D>, a, blocks, a.ksplit, W * 32,
-                            smem, stream, true);
+                            smem, stream, a.overlap != 0);
 }
 
 }  // namespace b200q

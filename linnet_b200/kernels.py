@@ -166,8 +166,8 @@ def int4_linear(x: torch.Tensor, packed: torch.Tensor, scale: torch.Tensor,
     weights at once (`B200Q_EARLY_DEPENDENTS`).  `swiglu` (eager calls only): `x` is
     [rows, 2 In] and the product's input is `silu(x[:, :In]) * x[:, In:]`, formed inside the
     product for one and two rows (`B200Q_SWIGLU_INPUT`) and by `glue.silu_mul` otherwise.
-    `overlap=False` (eager calls only): the one- and two-row kernel starts in plain stream order
-    instead of early (`B200Q_NO_OVERLAP`)."""
+    `overlap=False` (eager calls only): the kernel starts in plain stream order instead of early
+    (`B200Q_NO_OVERLAP`); weights that have to be copied here always do."""
     if out is None and not early and not swiglu and overlap and torch.compiler.is_compiling():
         return _int4_linear_op(x, packed, scale, zero)
     return _int4_linear(x, packed, scale, zero, out, early, swiglu, overlap)

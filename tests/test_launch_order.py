@@ -101,3 +101,33 @@ def test_int8_copied_weights_and_scales(rows):
         graph.replay()
         for y, ref in zip(captured, want):
             assert torch.equal(y, ref)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows", [1, 4, 12, 40])
+@pytest.mark.parametrize("group", [64, 128])
+def test_int4_copied_weights(rows, group):
+    """Strided packed weights, scales and zero points, through every kernel that few rows reach,
+    against the same product of tensors kept as they are."""
+    depth, out = 2048, 3000
+    gen = torch.Generator().manual_seed(rows + group)
+    inputs = torch.randn(rows, depth, generator=gen).to(torch.bfloat16).cuda()
+    kept, given = [], []
+    for _ in range(3):
+        packed = torch.randint(0, 256, (out, depth // group, group // 2), generator=gen, dtype=torch.uint8)
+        scale = (torch.rand(out, depth // group, generator=gen) * 0.02 + 1e-3).to(torch.bfloat16)
+        zero = torch.randint(0, 16, (out, depth // group), generator=gen, dtype=torch.uint8)
+        layer = [t.cuda() for t in (packed, scale, zero)]
+        kept.append(layer)
+        given.append([torch.stack((t, t), dim=-1)[..., 0] for t in layer])
+    assert not any(t.is_contiguous() for layer in given for t in layer)
+    want = [kernels.int4_linear(inputs, *layer) for layer in kept]
+    for y, ref in zip((kernels.int4_linear(inputs, *layer) for layer in given), want):
+        assert torch.equal(y, ref)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        captured = [kernels.int4_linear(inputs, *layer) for layer in given]
+    for _ in range(3):
+        graph.replay()
+        for y, ref in zip(captured, want):
+            assert torch.equal(y, ref)
