@@ -125,7 +125,8 @@ struct Pipe8 {
 
 // One finished accumulator: this thread's row m (a lane of tensor memory), bn columns from n0.
 __device__ __forceinline__ void store_tile(const MmArgs& a, uint32_t taddr, int m, int n0, int bn) {
-    const float xs = m < a.M ? __ldg(a.x_scale + m) : 0.0f;
+    // (written by the kernel ahead of this one, often to the address of an earlier layer's scales)
+    const float xs = m < a.M ? ld_mutable(a.x_scale + m) : 0.0f;
 #pragma unroll 1
     for (int c0 = 0; c0 < bn; c0 += 32) {
         uint32_t v[32];

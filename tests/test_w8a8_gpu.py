@@ -104,3 +104,39 @@ def test_int8_group_linear_many_rows(rows):
     want = lo.int8_group_linear(x, q, scale).float()
     got = quantized.int8_group_linear(x.cuda(), quantized.int8_group_operands(q.cuda(), scale.cuda()), None)
     torch.testing.assert_close(got.float().cpu(), want, rtol=1e-2, atol=1e-2)
+
+
+@pytest.mark.parametrize("rows", [100, 600])
+def test_layers_of_a_graph_share_the_scale_buffer(rows):
+    """Rounding and product of several layers over one pair of buffers, as the allocator hands them
+    out inside a captured pass: every product takes its own layer's scales (one-block kernel and
+    pairs)."""
+    from linnet_b200 import _lib, kernels
+
+    lib = _lib.load()
+    depth, out, layers = 512, 4096, 4
+    gen = torch.Generator().manual_seed(rows)
+    w = torch.randint(-127, 128, (out, depth), generator=gen, dtype=torch.int8).cuda()
+    ws = (torch.rand(out, generator=gen) * 0.01 + 1e-4).cuda()
+    xs = [(torch.randn(rows, depth, generator=gen) * 10.0 ** i).to(torch.bfloat16).cuda() for i in range(layers)]
+    want = []
+    for x in xs:
+        levels, scales = kernels.int8_rows(x)
+        torch.cuda.synchronize()
+        want.append(kernels.int8_mm(levels, w, scales, ws, torch.bfloat16))
+        torch.cuda.synchronize()
+    q = torch.empty(rows, depth, dtype=torch.int8, device="cuda")
+    s = torch.empty(rows, 1, dtype=torch.float32, device="cuda")
+    ys = [torch.zeros(rows, out, dtype=torch.bfloat16, device="cuda") for _ in xs]
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        stream = torch.cuda.current_stream().cuda_stream
+        for x, y in zip(xs, ys):
+            _lib.check(lib.b200q_int8_rows(x.data_ptr(), q.data_ptr(), s.data_ptr(), rows, depth, _lib.BF16, stream))
+            _lib.check(lib.b200q_int8_mm(q.data_ptr(), w.data_ptr(), s.data_ptr(), ws.data_ptr(), y.data_ptr(), rows,
+                                         depth, out, _lib.BF16, stream))
+    for _ in range(5):
+        graph.replay()
+        torch.cuda.synchronize()
+        for y, ref in zip(ys, want):
+            assert torch.equal(y, ref)
