@@ -99,3 +99,56 @@ def test_wait_limit_argument_is_checked():
     lib = _lib.load()
     assert lib.b200q_set_wait_limit_ns(0) == _lib.ERROR
     assert "between 1 ns and 60 s" in _lib.last_error()
+
+
+@pytest.mark.parametrize(("bits", "rows"), [(4, 1), (4, 16), (4, 100), (8, 1), (8, 40)])
+def test_products_outlast_a_slow_rank(bits, rows):
+    """A reduction may wait longer for its peers (1.5 s here) than a product's own bounded waits
+    last (about a second).  The product launched behind it starts early, but its waits do not run
+    while the reduction still waits: it finishes, and its result is right."""
+    from linnet_b200 import _lib, kernels
+
+    lib = _lib.load()
+    dev = torch.device("cuda", 0)
+    depth, out, world = 4096, 4096, 2
+    gen = torch.Generator().manual_seed(rows)
+    x = torch.randn(rows, depth, generator=gen).to(torch.bfloat16).cuda()
+    if bits == 4:
+        weight = (torch.randint(0, 256, (out, depth // 128, 64), generator=gen, dtype=torch.uint8).cuda(),
+                  (torch.rand(out, depth // 128, generator=gen) * 0.02 + 1e-3).to(torch.bfloat16).cuda(),
+                  torch.randint(0, 16, (out, depth // 128), generator=gen, dtype=torch.uint8).cuda())
+
+        def product() -> torch.Tensor:
+            return kernels.int4_linear(x, *weight)
+    else:
+        weight = (torch.randint(-128, 128, (out, depth), generator=gen, dtype=torch.int8).cuda(),
+                  (torch.rand(out, generator=gen) * 0.01 + 1e-4).cuda())
+
+        def product() -> torch.Tensor:
+            return (kernels.gemv8 if rows == 1 else kernels.w8a16)(x, *weight, False, 0, 1)
+
+    want = product()
+    state = torch.zeros(3, dtype=torch.int32, device=dev)
+    slot_words = ROWS * HIDDEN // 2
+    areas = [torch.zeros(world, slot_words, 2, dtype=torch.int32, device=dev) for _ in range(world)]
+    area_ptrs = (ctypes.c_int64 * world)(*[a.data_ptr() for a in areas])
+    residual = torch.zeros(ROWS, HIDDEN, dtype=torch.bfloat16, device=dev)
+    partial, y = torch.ones_like(residual), torch.empty_like(residual)
+    norm = torch.ones(HIDDEN, device=dev, dtype=torch.bfloat16)
+    torch.cuda.synchronize()
+    _lib.check(lib.b200q_int4_gemm_status())
+    _lib.check(lib.b200q_set_wait_limit_ns(1_500_000_000))
+    try:
+        t0 = time.perf_counter()
+        _lib.check(lib.b200q_tp_allreduce_add_rmsnorm(
+            ctypes.addressof(area_ptrs), slot_words, partial.data_ptr(), world, 0, state.data_ptr(),
+            state.data_ptr() + 4, state.data_ptr() + 8, residual.data_ptr(), norm.data_ptr(), y.data_ptr(), ROWS, HIDDEN,
+            1e-5, _stream()))
+        got = product()
+        torch.cuda.synchronize()
+        assert time.perf_counter() - t0 > 1.4, "the reduction should have waited for its limit"
+    finally:
+        _lib.check(lib.b200q_set_wait_limit_ns(1_000_000_000))
+    assert int(state[2]) == 101
+    _lib.check(lib.b200q_int4_gemm_status())
+    assert torch.equal(got, want)
