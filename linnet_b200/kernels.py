@@ -302,6 +302,40 @@ def w8a16_any_rows(x: torch.Tensor, weight: torch.Tensor, scale: torch.Tensor, g
             and scale.dtype == torch.float32 and scale.is_contiguous() and scale.data_ptr() % 16 == 0)
 
 
+def _w8a16_many(x: torch.Tensor, weight: torch.Tensor, scale: torch.Tensor, group: int) -> torch.Tensor:
+    if w8a16_any_rows(x, weight, scale, group):
+        return _eight_bit("w8a16", x, weight, scale, False, group, 1)
+    dequantized = dequantize8(weight, scale, False, group, 1, x.dtype)
+    # f32 accumulation all the way: the library may otherwise add split-K partial sums in the
+    # 16-bit type, which alone costs more than the 1e-2 this layer is held to.
+    matmul = torch.backends.cuda.matmul
+    saved = (matmul.allow_bf16_reduced_precision_reduction, matmul.allow_fp16_reduced_precision_reduction)
+    matmul.allow_bf16_reduced_precision_reduction = matmul.allow_fp16_reduced_precision_reduction = False
+    try:
+        return torch.nn.functional.linear(x, dequantized)
+    finally:
+        matmul.allow_bf16_reduced_precision_reduction, matmul.allow_fp16_reduced_precision_reduction = saved
+
+
+@torch.library.custom_op("linnet::w8a16_many", mutates_args=(), device_types="cuda")
+def _w8a16_many_op(x: torch.Tensor, weight: torch.Tensor, scale: torch.Tensor, group: int) -> torch.Tensor:
+    return _w8a16_many(x, weight, scale, group)
+
+
+@_w8a16_many_op.register_fake
+def _(x, weight, scale, group):
+    return x.new_empty(x.shape[0], weight.shape[0])
+
+
+def w8a16_many(x: torch.Tensor, weight: torch.Tensor, scale: torch.Tensor, group: int) -> torch.Tensor:
+    """`F.linear(x, W)` for more rows than `w8a16` is tiled for: the tensor-core product where
+    `w8a16_any_rows` says so, else `dequantize8` and the library product.  One op under
+    `torch.compile`: the choice looks at addresses, which a trace does not have."""
+    if torch.compiler.is_compiling():
+        return _w8a16_many_op(x, weight, scale, group)
+    return _w8a16_many(x, weight, scale, group)
+
+
 def dequantize8(weight: torch.Tensor, scale: torch.Tensor, fp8: bool, group: int, row_block: int,
                 dtype: torch.dtype) -> torch.Tensor:
     """The int8 weight of `gemv8` dequantized to `dtype` (f32 product, one rounding)."""

@@ -6,10 +6,10 @@ per step.  The operand tuples have the reference's members
 (`Int8Operands = (weight, scale_f32, rounded, fast)`, quantized.py:62-66).
 
 Row-count dispatch as the reference's `_weight_only` (quantized.py:90-105): one row goes to
-`gemv8`, more rows to `w8a16`, whose tensor-core kernel dequantizes the weight inside the product
-at any row count.  Shapes that kernel does not take (`kernels.w8a16_any_rows`) keep the
-reference's route from `TILED_ROWS` rows on: the weight dequantized once with `dequantize8` and
-the dense product handed to the library GEMM.  `rounded` with more than `FEW_ROWS` rows takes the
+`gemv8`, up to `TILED_ROWS` rows to `w8a16`, more to `w8a16_many`, whose tensor-core kernel
+dequantizes the weight inside the product.  Shapes that kernel does not take
+(`kernels.w8a16_any_rows`) keep the reference's route there: the weight dequantized once with
+`dequantize8` and the dense product handed to the library GEMM.  `rounded` with more than `FEW_ROWS` rows takes the
 8-bit-activation route (`int8_rows` + `int8_mm`, quantized.py:187-189).  There is no fallback for
 CPU tensors.
 """
@@ -34,18 +34,9 @@ def _weight_only(flat: torch.Tensor, weight: torch.Tensor, scale: torch.Tensor, 
     rows = flat.shape[0]
     if rows == 1:
         return kernels.gemv8(flat, weight, scale, False, group, 1)
-    if rows <= TILED_ROWS or kernels.w8a16_any_rows(flat, weight, scale, group):
+    if rows <= TILED_ROWS:
         return kernels.w8a16(flat, weight, scale, False, group, 1)
-    dequantized = kernels.dequantize8(weight, scale, False, group, 1, flat.dtype)
-    # f32 accumulation all the way: the library may otherwise add split-K partial sums in the
-    # 16-bit type, which alone costs more than the 1e-2 this layer is held to.
-    matmul = torch.backends.cuda.matmul
-    saved = (matmul.allow_bf16_reduced_precision_reduction, matmul.allow_fp16_reduced_precision_reduction)
-    matmul.allow_bf16_reduced_precision_reduction = matmul.allow_fp16_reduced_precision_reduction = False
-    try:
-        return torch.nn.functional.linear(flat, dequantized)
-    finally:
-        matmul.allow_bf16_reduced_precision_reduction, matmul.allow_fp16_reduced_precision_reduction = saved
+    return kernels.w8a16_many(flat, weight, scale, group)
 
 
 def _finish(x: torch.Tensor, y: torch.Tensor, bias: torch.Tensor | None) -> torch.Tensor:
