@@ -16,6 +16,7 @@ their arguments.  There is no fallback: tensors must live on a B200.
 from __future__ import annotations
 
 import torch
+from torch.autograd import forward_ad
 
 from . import _lib
 
@@ -305,6 +306,10 @@ def w8a16_any_rows(x: torch.Tensor, weight: torch.Tensor, scale: torch.Tensor, g
 def _w8a16_many(x: torch.Tensor, weight: torch.Tensor, scale: torch.Tensor, group: int) -> torch.Tensor:
     if w8a16_any_rows(x, weight, scale, group):
         return _eight_bit("w8a16", x, weight, scale, False, group, 1)
+    return _dense8(x, weight, scale, group)
+
+
+def _dense8(x: torch.Tensor, weight: torch.Tensor, scale: torch.Tensor, group: int) -> torch.Tensor:
     dequantized = dequantize8(weight, scale, False, group, 1, x.dtype)
     # f32 accumulation all the way: the library may otherwise add split-K partial sums in the
     # 16-bit type, which alone costs more than the 1e-2 this layer is held to.
@@ -330,9 +335,15 @@ def _(x, weight, scale, group):
 def w8a16_many(x: torch.Tensor, weight: torch.Tensor, scale: torch.Tensor, group: int) -> torch.Tensor:
     """`F.linear(x, W)` for more rows than `w8a16` is tiled for: the tensor-core product where
     `w8a16_any_rows` says so, else `dequantize8` and the library product.  One op under
-    `torch.compile`: the choice looks at addresses, which a trace does not have."""
+    `torch.compile`: the choice looks at addresses, which a trace does not have.  Rows that are
+    differentiated or batched (autograd, forward mode, `torch.func`) take the library product,
+    which PyTorch knows the derivatives of."""
+    if torch.is_grad_enabled() and x.requires_grad:
+        return _dense8(x, weight, scale, group)
     if torch.compiler.is_compiling():
         return _w8a16_many_op(x, weight, scale, group)
+    if torch._C._functorch.is_functorch_wrapped_tensor(x) or forward_ad.unpack_dual(x).tangent is not None:
+        return _dense8(x, weight, scale, group)
     return _w8a16_many(x, weight, scale, group)
 
 
