@@ -29,6 +29,7 @@
 #include "int4_gemv_oct.cuh"
 #include "int4_gemv_tma.cuh"
 #include "int4_gemv_rows.cuh"
+#include "wq_gemm.cuh"
 
 namespace b200q {
 namespace {
@@ -318,9 +319,13 @@ int32_t dispatch_gemv(const GemvArgs& a, const Plan& p, cudaStream_t stream) {
 // Three or more rows: the kernel that stages the activations once per block.  Picks the
 // warps (tiles) per block so that every block of the grid is resident at once, and the
 // octs per block so that the cluster has at most 8 blocks.
+bool rows_kernel_takes(const GemvArgs& a) {
+    return a.G == 128 && a.K % 1024 == 0 && aligned(a.scale, 16) && aligned(a.zero, 8);
+}
+
 template <typename T, int MB>
 bool run_rows(const GemvArgs& a, cudaStream_t stream, int32_t* status) {
-    if (a.G != 128 || a.K % 1024 != 0 || !aligned(a.scale, 16) || !aligned(a.zero, 8)) return false;
+    if (!rows_kernel_takes(a)) return false;
     const int octs = a.K / 1024;
     int opc = 0;
     for (int c = 1; c <= octs; ++c)
@@ -438,6 +443,7 @@ struct NormInput {  // the input of the product is rms_norm(x + delta) * weight
     float eps;
 };
 
+// Without `status`: only says whether it takes the call.
 template <typename T>
 bool run_tma(const GemvArgs& a, cudaStream_t stream, int32_t* status, const NormInput* norm = nullptr) {
     if (a.G != 128 || a.M > 2 || size_t(a.N) * size_t(a.K / 2) >= (size_t(1) << 40)) return false;
@@ -451,6 +457,7 @@ bool run_tma(const GemvArgs& a, cudaStream_t stream, int32_t* status, const Norm
     TmaArgs half = p;  // items of half the size: twice the warps a tile
     size_t smem = 0, half_smem = 0;
     const bool whole = tma_plan<1, 16, 8>(p, a.G, &smem), halves = tma_plan<1, 16, 4>(half, a.G, &half_smem);
+    if (status == nullptr) return halves || whole;
     if (halves && (!whole || half_items_pay(half, sms))) {
         *status = launch_tma<T, 1, 16, 4, false>(half, a.packed, half_smem, sms, stream);
         return true;
@@ -510,6 +517,19 @@ int32_t run_gemv(GemvArgs a, int64_t rows, cudaStream_t stream) {
 }
 
 }  // namespace
+
+int64_t int4_unrounded_rows(const WqProblem& p, int32_t flags) {
+    if (flags & B200Q_EXACT_WEIGHTS) return 0;
+    GemvArgs a{p.x, static_cast<const uint8_t*>(p.weight), p.scale, p.zero, p.y, 0, int(p.in), int(p.out), int(p.group),
+               int(p.in / 128), 0, 1, flags};
+    // bf16 prompts, whose weights are rounded whatever the row count
+    if (p.dtype == B200Q_BF16 && p.rows > 32 && p.out * (p.in / 2) < (int64_t(1) << 32)) return 0;
+    const int64_t pass = rows_kernel_takes(a) ? 64 : 16;
+    a.M = p.rows > pass ? int(p.rows % pass) : 0;
+    if (a.M < 1 || a.M > 2) return 0;
+    const bool taken = p.dtype == B200Q_BF16 ? run_tma<__nv_bfloat16>(a, nullptr, nullptr) : run_tma<__half>(a, nullptr, nullptr);
+    return taken ? a.M : 0;
+}
 
 int32_t check_int4_args(const char* who, const void* x, const uint8_t* packed, const void* scale,
                         const uint8_t* zero, void* y, int64_t rows, int64_t in, int64_t out,

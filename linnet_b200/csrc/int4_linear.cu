@@ -48,11 +48,22 @@ extern "C" int32_t b200q_int4_linear_ex(const void* x, const uint8_t* packed, co
     if (rows >= gemm_rows(in, out, group) && !(flags & B200Q_SWIGLU_INPUT)) {
         const int32_t ok = check_int4_args("int4_linear", x, packed, scale, zero, y, rows, in, out, group, dtype);
         if (ok != B200Q_OK) return ok;
-        const WqProblem p{kWqInt4, x, packed, scale, zero, y, rows, in, out, group, dtype};
+        WqProblem p{kWqInt4, x, packed, scale, zero, y, rows, in, out, group, dtype};
         const WqStart start = (flags & B200Q_NO_OVERLAP) ? WqStart::kStreamOrder
                               : rows <= kOverlapRows     ? WqStart::kFetchAhead
                                                          : WqStart::kEarly;
-        if (wq_gemm_supports(p)) return wq_gemm("int4_linear", p, start, static_cast<cudaStream_t>(stream));
+        // One or two rows past the passes of the decode kernels stay with the kernel that takes their
+        // zero points and scales unrounded: a second launch, and sums with the smaller error.
+        const int64_t last = int4_unrounded_rows(p, flags), first = rows - last;
+        if (last == 0 || first >= gemm_rows(in, out, group)) {
+            p.rows = first;
+            if (wq_gemm_supports(p)) {
+                const int32_t status = wq_gemm("int4_linear", p, start, static_cast<cudaStream_t>(stream));
+                if (status != B200Q_OK || last == 0) return status;
+                return b200q_int4_gemv_ex(static_cast<const uint16_t*>(x) + first * in, packed, scale, zero,
+                                          static_cast<uint16_t*>(y) + first * out, last, in, out, group, dtype, flags, stream);
+            }
+        }
     }
     return b200q_int4_gemv_ex(x, packed, scale, zero, y, rows, in, out, group, dtype, flags, stream);
 }

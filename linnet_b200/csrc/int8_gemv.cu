@@ -266,7 +266,8 @@ int32_t dispatch_gemv8(const Gemv8Args& a, cudaStream_t stream) {
 
 // One scale a row, one or two activation rows, and no request for the per-weight rounding:
 // the kernel of int8_gemv_tma.cuh, which applies the scale to the finished sum as the
-// reference's own GPU kernel does (python/linnet/src/linnet/torch/kernels.py:352-371).
+// reference's own GPU kernel does (python/linnet/src/linnet/torch/kernels.py:352-371).  Without
+// `status`: only says whether it takes the call.
 template <typename T>
 bool run_tma8(const Gemv8Args& a, cudaStream_t stream, int32_t* status) {
     if ((a.G != 0 && a.G != a.K) || a.M > 2 || (a.flags & B200Q_EXACT_WEIGHTS)) return false;
@@ -279,6 +280,7 @@ bool run_tma8(const Gemv8Args& a, cudaStream_t stream, int32_t* status) {
     Tma8Args half = p;  // items of half the size: twice the warps a tile
     size_t smem = 0, half_smem = 0;
     const bool whole = tma8_plan<16, 8>(p, &smem), halves = tma8_plan<16, 4>(half, &half_smem);
+    if (status == nullptr) return halves || whole;
     if (halves && (!whole || half_items_pay(half, sms) || half.producers > p.producers)) {
         *status = launch_tma8<T, 16, 4>(half, a.w, half_smem, sms, stream);
         return true;
@@ -308,17 +310,27 @@ int64_t gemm_rows8(int64_t weights) {
 
 template <typename T>
 int32_t run_gemv8(Gemv8Args a, int64_t rows, cudaStream_t stream) {
+    const uint8_t* x = static_cast<const uint8_t*>(a.x);
+    uint8_t* y = static_cast<uint8_t*>(a.y);
+    int64_t done = 0;
     if (rows >= gemm_rows8(int64_t(a.K) * a.N)) {
+        // One or two rows past a multiple of 16 stay with the kernel that takes their scales
+        // unrounded, as in the passes below: a second launch, and sums with the smaller error.
+        a.M = rows > 16 ? int(rows % 16) : 0;
+        const int64_t last = a.M >= 1 && a.M <= 2 && run_tma8<T>(a, stream, nullptr) ? a.M : 0;
         // the same weights as the decode kernel's below: scaled in f32, rounded once
-        const WqProblem p{kWqInt8, a.x, a.w, a.scale, nullptr, a.y, rows, a.K, a.N, a.G == 0 ? a.K : a.G, Half16<T>::kDtype};
+        const WqProblem p{kWqInt8, x, a.w, a.scale, nullptr, y, rows - last, a.K, a.N, a.G == 0 ? a.K : a.G,
+                          Half16<T>::kDtype};
         const WqStart start = (a.flags & B200Q_NO_OVERLAP) ? WqStart::kStreamOrder
                               : rows <= kOverlapRows8      ? WqStart::kFetchAhead
                                                            : WqStart::kEarly;
-        if (wq_gemm_supports(p)) return wq_gemm("int8_linear", p, start, stream);
+        if (wq_gemm_supports(p)) {
+            const int32_t status = wq_gemm("int8_linear", p, start, stream);
+            if (status != B200Q_OK) return status;
+            done = p.rows;
+        }
     }
-    const uint8_t* x = static_cast<const uint8_t*>(a.x);
-    uint8_t* y = static_cast<uint8_t*>(a.y);
-    for (int64_t m0 = 0; m0 < rows; m0 += 16) {
+    for (int64_t m0 = done; m0 < rows; m0 += 16) {
         a.M = int(rows - m0 < 16 ? rows - m0 : 16);
         a.x = x + size_t(m0) * a.K * 2;
         a.y = y + size_t(m0) * a.N * 2;

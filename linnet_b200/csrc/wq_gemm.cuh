@@ -29,4 +29,8 @@ enum class WqStart {
 };
 int32_t wq_gemm(const char* who, const WqProblem& p, WqStart start, cudaStream_t stream);
 
+// int4_gemv.cu: of this many rows, how many at the end the decode kernels' passes of 16 (or 64) leave
+// to the one- and two-row kernel, whose sums take zero point and scale unrounded.
+int64_t int4_unrounded_rows(const WqProblem& p, int32_t flags);
+
 }  // namespace b200q

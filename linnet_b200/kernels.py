@@ -227,7 +227,7 @@ def _no_fp8(who: str, fp8: bool) -> None:
 
 
 def _eight_bit(who: str, x: torch.Tensor, weight: torch.Tensor, scale: torch.Tensor, fp8: bool,
-               group: int, row_block: int) -> torch.Tensor:
+               group: int, row_block: int, rounded: bool = False) -> torch.Tensor:
     _no_fp8(who, fp8)
     if row_block != 1:
         raise NotImplementedError(f"{who}: block scales (row_block {row_block}) are an FP8 format")
@@ -243,7 +243,7 @@ def _eight_bit(who: str, x: torch.Tensor, weight: torch.Tensor, scale: torch.Ten
     scale = scale.float().contiguous()
     # copied just now: no fetch of them ahead of the kernel that writes them
     copied = weight is not given[0] or scale is not given[1]
-    flags = (_lib.EXACT_WEIGHTS if _exact_weights else 0) | (_lib.NO_OVERLAP if copied else 0)
+    flags = (_lib.EXACT_WEIGHTS if _exact_weights or rounded else 0) | (_lib.NO_OVERLAP if copied else 0)
     y = torch.empty(rows, width, dtype=x.dtype, device=device)
     with _Device(device):
         _lib.check(_lib.load().b200q_int8_linear_ex(
@@ -305,7 +305,7 @@ def w8a16_any_rows(x: torch.Tensor, weight: torch.Tensor, scale: torch.Tensor, g
 
 def _w8a16_many(x: torch.Tensor, weight: torch.Tensor, scale: torch.Tensor, group: int) -> torch.Tensor:
     if w8a16_any_rows(x, weight, scale, group):
-        return _eight_bit("w8a16", x, weight, scale, False, group, 1)
+        return _eight_bit("w8a16", x, weight, scale, False, group, 1, rounded=True)
     return _dense8(x, weight, scale, group)
 
 
@@ -333,7 +333,8 @@ def _(x, weight, scale, group):
 
 
 def w8a16_many(x: torch.Tensor, weight: torch.Tensor, scale: torch.Tensor, group: int) -> torch.Tensor:
-    """`F.linear(x, W)` for more rows than `w8a16` is tiled for: the tensor-core product where
+    """`F.linear(x, W)` for more rows than `w8a16` is tiled for, every weight rounded to the type of
+    `x` as `dequantize8` rounds it: the tensor-core product where
     `w8a16_any_rows` says so, else `dequantize8` and the library product.  One op under
     `torch.compile`: the choice looks at addresses, which a trace does not have.  Rows that are
     differentiated or batched (autograd, forward mode, `torch.func`) take the library product,

@@ -116,3 +116,42 @@ def test_unaligned_activations_keep_the_library_route():
     assert not kernels.w8a16_any_rows(inner, operands[0], operands[1], 0)
     got = quantized.int8_linear(inner, operands, None)
     check(got, x[1:].view(100, 512), lo.int8_weight(weight, scale.reshape(-1), torch.bfloat16))
+
+
+@pytest.mark.parametrize(("rows", "depth", "out", "dtype"), [
+    (17, 1536, 4096, torch.bfloat16), (18, 5632, 1000, torch.bfloat16), (33, 1536, 4096, torch.float16),
+    (50, 2560, 4096, torch.float16), (65, 2048, 4096, torch.float16), (130, 4096, 4096, torch.float16),
+])
+def test_int4_rows_past_the_passes_keep_unrounded_weights(rows, depth, out, dtype):
+    """The one or two rows that passes of the decode kernels leave over come from the one- and
+    two-row kernel, bit for bit, which takes zero points and scales unrounded."""
+    from linnet_b200 import kernels
+
+    gen = torch.Generator().manual_seed(rows + depth)
+    packed, scale, zero = (t.cuda() for t in make_int4(out, depth, 128, dtype, gen, 0.02))
+    x = torch.randn(rows, depth, generator=gen).to(dtype).cuda()
+    last = rows % 16
+    got = kernels.int4_linear(x, packed, scale, zero)
+    assert torch.equal(got[-last:], kernels.int4_linear(x[-last:], packed, scale, zero))
+    check(got[:-last], x[:-last].cpu(), lo.int4_weight(packed.cpu(), scale.cpu(), zero.cpu(), dtype))
+
+
+@pytest.mark.parametrize(("rows", "dtype"), [(17, torch.bfloat16), (18, torch.float16), (33, torch.float16),
+                                             (34, torch.bfloat16), (50, torch.bfloat16), (66, torch.bfloat16)])
+def test_int8_rows_past_the_passes_keep_unrounded_weights(rows, dtype):
+    """The same for int8 with one scale a row, at any row count of `w8a16`; an int8 layer past the
+    rows `w8a16` is tiled for rounds every weight, as its dense route does."""
+    from linnet_b200 import kernels, quantized
+
+    depth, out = 4096, 3000
+    gen = torch.Generator().manual_seed(rows)
+    weight, scale = make_int8(out, depth, 0, gen)
+    x = torch.randn(rows, depth, generator=gen).to(dtype)
+    w, s, rounded = weight.cuda(), scale.reshape(-1).cuda(), lo.int8_weight(weight, scale.reshape(-1), dtype)
+    last = rows % 16
+    got = kernels.w8a16(x.cuda(), w, s, False, 0, 1)
+    few = kernels.gemv8 if last == 1 else kernels.w8a16
+    assert torch.equal(got[-last:], few(x[-last:].cuda(), w, s, False, 0, 1))
+    check(got[:-last], x[:-last], rounded)
+    if rows > quantized.TILED_ROWS:
+        check(quantized.int8_linear(x.cuda(), quantized.int8_operands(w, s, 0), None), x, rounded)
