@@ -102,7 +102,8 @@ int32_t b200q_int4_gemv(const void* x, const uint8_t* packed, const void* scale,
  *     their own wait on this one's results) as soon as this one has started, instead of
  *     when its last weights are in: pays when the next kernel is another product that can
  *     prefetch its weights meanwhile (q, k, v of one input; a chain of products), costs
- *     when the next kernel only takes room while it waits.
+ *     when the next kernel only takes room while it waits.  For the decode kernels: the
+ *     tensor-core product always lets the next kernel start at once.
  *   B200Q_SWIGLU_INPUT   x is [rows, 2 in]: the product's input is silu(x[:, :in]) * x[:, in:]
  *     (silu rounded to the 16-bit type, then the product rounded, as the two PyTorch ops of the
  *     reference's generated source do), formed while the kernel stages its activations: the

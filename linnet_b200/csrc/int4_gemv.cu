@@ -558,8 +558,7 @@ extern "C" int32_t b200q_int4_gemv_ex(const void* x, const uint8_t* packed, cons
                                       void* stream) {
     const int32_t ok = check_int4_args("int4_gemv", x, packed, scale, zero, y, rows, in, out, group, dtype);
     if (ok != B200Q_OK || rows == 0) return ok;
-    B200Q_REQUIRE((flags & ~(B200Q_EXACT_WEIGHTS | B200Q_EARLY_DEPENDENTS | B200Q_SWIGLU_INPUT | B200Q_NO_OVERLAP)) == 0,
-                  "int4_gemv: unknown flag bits %d", flags);
+    B200Q_REQUIRE((flags & ~kInt4Flags) == 0, "int4_gemv: unknown flag bits %d", flags);
     GemvArgs a{x, packed, scale, zero, y, 0, int(in), int(out), int(group), int(in / 128), 0, 1, flags};
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (flags & B200Q_SWIGLU_INPUT) {

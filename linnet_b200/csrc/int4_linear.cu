@@ -48,6 +48,7 @@ extern "C" int32_t b200q_int4_linear_ex(const void* x, const uint8_t* packed, co
     if (rows >= gemm_rows(in, out, group) && !(flags & B200Q_SWIGLU_INPUT)) {
         const int32_t ok = check_int4_args("int4_linear", x, packed, scale, zero, y, rows, in, out, group, dtype);
         if (ok != B200Q_OK) return ok;
+        B200Q_REQUIRE((flags & ~kInt4Flags) == 0, "int4_linear: unknown flag bits %d", flags);
         WqProblem p{kWqInt4, x, packed, scale, zero, y, rows, in, out, group, dtype};
         const WqStart start = (flags & B200Q_NO_OVERLAP) ? WqStart::kStreamOrder
                               : rows <= kOverlapRows     ? WqStart::kFetchAhead

@@ -6,6 +6,9 @@
 
 namespace b200q {
 
+// What b200q_int4_gemv_ex and b200q_int4_linear_ex take, whichever kernel serves the call.
+constexpr int32_t kInt4Flags = B200Q_EXACT_WEIGHTS | B200Q_EARLY_DEPENDENTS | B200Q_SWIGLU_INPUT | B200Q_NO_OVERLAP;
+
 enum WqFormat { kWqInt4 = 0, kWqInt8 = 1 };
 
 struct WqProblem {

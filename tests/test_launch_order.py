@@ -60,6 +60,16 @@ def test_int8_entry_takes_the_flag():
     assert lib.b200q_int8_linear_ex(*arguments, 1 << 10, None) == _lib.ERROR
 
 
+@pytest.mark.parametrize("rows", [1, 12, 40])
+def test_int4_entry_refuses_unknown_flags(rows):
+    """Whatever kernel would serve the call; refused before any launch."""
+    lib = _lib.load()
+    address = 1 << 12
+    assert lib.b200q_int4_linear_ex(address, address, address, address, address, rows, 64, 32, 64, _lib.BF16, 1 << 10,
+                                    None) == _lib.ERROR
+    assert "unknown flag bits" in _lib.last_error()
+
+
 def int8_layer(depth, out, seed):
     gen = torch.Generator().manual_seed(seed)
     weight = torch.randint(-127, 128, (out, depth), generator=gen, dtype=torch.int8)
