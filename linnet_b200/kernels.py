@@ -41,8 +41,8 @@ def _on_gpu(who: str, *tensors: torch.Tensor) -> torch.device:
 
 # PyTorch's own accessors, without the Stream object and the initialisation check that
 # `torch.cuda.current_stream` and `current_device` go through: a one-row call is bound by its host path.
-_raw_stream = torch._C._cuda_getCurrentRawStream
-_current_device = torch._C._cuda_getDevice
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)  # None: a PyTorch without CUDA
+_current_device = getattr(torch._C, "_cuda_getDevice", None)
 
 
 def _stream(device: torch.device) -> int:

@@ -86,3 +86,17 @@ def test_ops_refuse_cpu_tensors():
     with pytest.raises(ValueError, match="a group of 24 is not 16, 32, 64, or a multiple of 128"):
         kernels.int4_linear(torch.zeros(1, 24, dtype=torch.bfloat16),
                             torch.zeros(16, 1, 12, dtype=torch.uint8), scale, zero)
+
+
+def test_package_imports_without_cuda_accessors():
+    """A CPU-only PyTorch has none of the `torch._C._cuda_*` accessors: the modules still import
+    (checkpoints can be read and written there), and only a launch needs them."""
+    import subprocess
+    import sys
+
+    code = ("import torch\n"
+            "for name in [n for n in dir(torch._C) if n.startswith('_cuda_')]: delattr(torch._C, name)\n"
+            "import linnet_b200.kernels, linnet_b200.quantized, linnet_b200.int4, linnet_b200.checkpoint\n"
+            "import linnet_b200.glue, linnet_b200.decoder, linnet_b200.backend, linnet_b200.tp\n")
+    done = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True)
+    assert done.returncode == 0, done.stderr
