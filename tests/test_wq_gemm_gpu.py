@@ -1,7 +1,7 @@
 """The tensor-core product of 16-bit activations and quantized weights at the sizes where it can go
 wrong: one row to several tiles of rows, K that ends in half an item (64 of 128 inputs), one item
-only, ragged N, K split over a cluster, one and two accumulators, every group size it takes, both
-16-bit types, scales at the ends of their range."""
+a tile, ragged N, every group size it takes, both 16-bit types, scales at the ends of their range,
+values that are not finite."""
 
 from __future__ import annotations
 
@@ -53,9 +53,9 @@ def test_int4_weights_are_exact(dtype, group):
         assert torch.equal(got.t().cpu().float(), want.float())
 
 
-# (rows, depth, out): the plans these reach are one item; a last item of half; a K split of four;
-# two tiles a block with two accumulators; two blocks of rows a tile; one accumulator (rows 200, 256);
-# several tiles of rows with a ragged last one
+# (rows, depth, out): few rows (the smallest stay with the decode kernels), a last item of half, wide
+# and narrow weights, short and long K, several tiles of rows with a ragged last one.  Which tile shape
+# and K split a size gets is the cost model's choice.
 SHAPES = [(1, 64, 128), (9, 128, 100), (17, 192, 1000), (33, 4160, 130), (64, 4096, 512), (16, 1024, 28680),
           (100, 320, 20000), (200, 448, 3000), (256, 1088, 4096), (257, 640, 5000), (1000, 256, 9001)]
 
@@ -87,6 +87,65 @@ def test_int8_product(rows, depth, out, group, dtype):
     else:
         got = quantized.int8_linear(x.cuda(), quantized.int8_operands(weight.cuda(), scale.cuda(), 0), None)
     check(got, x, lo.int8_weight(weight, scale if group else scale.reshape(-1), dtype))
+
+
+# One item of half or whole size a tile, for one tile in all and for three and more tiles a block, so
+# that a tile's single item falls to either issuer and accumulator.
+ONE_ITEM = [(16, 64, 128), (16, 128, 100), (16, 64, 60000), (16, 128, 60000), (16, 128, 75001), (40, 64, 57000),
+            (70, 128, 60000), (200, 128, 60000), (256, 64, 58000)]
+
+
+@pytest.mark.parametrize(("rows", "depth", "out"), ONE_ITEM)
+@pytest.mark.parametrize(("group", "dtype"), [(64, torch.bfloat16), (16, torch.float16)])
+def test_int4_one_item_a_tile(rows, depth, out, group, dtype):
+    test_int4_product(rows, depth, out, group, dtype)
+
+
+@pytest.mark.parametrize(("rows", "depth", "out"), ONE_ITEM)
+@pytest.mark.parametrize(("group", "dtype"), [(0, torch.float16), (64, torch.bfloat16), (16, torch.bfloat16)])
+def test_int8_one_item_a_tile(rows, depth, out, group, dtype):
+    test_int8_product(rows, depth, out, group, dtype)
+
+
+@pytest.mark.parametrize("group", [16, 48 * 16, 0])
+def test_int8_groups(group):
+    """The smallest group, one that is no power of two, and one scale a row, over a K that ends in half
+    an item."""
+    for rows in (16, 33, 150):
+        test_int8_product(rows, 768 * 3 + (0 if group > 16 else 64), 1500, group, torch.bfloat16)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("rows", [20, 80])
+def test_infinities_and_nan_stay_where_they_are(rows, dtype):
+    """An activation that is not finite makes its own row not finite, a scale its own column; every
+    other result is as without them."""
+    from linnet_b200 import kernels
+
+    depth, out, group = 512, 700, 64
+    gen = torch.Generator().manual_seed(rows)
+    packed, scale, zero = make_int4(out, depth, group, dtype, gen, 0.02)
+    zero = zero.clamp(max=14)  # a level equal to the zero point would make 0 times infinity
+    packed |= 0xFF             # every level is 15
+    weight, scale8 = make_int8(out, depth, group, gen)
+    weight = weight.clamp(min=1)
+    x = torch.randn(rows, depth, generator=gen).to(dtype)
+    odd, odd4, odd8 = x.clone(), scale.clone(), scale8.clone()
+    odd[3, 5], odd[7, 100] = float("inf"), float("nan")
+    odd4[11, 2], odd4[600, 0] = float("inf"), float("nan")
+    odd8[11, 2], odd8[600, 0] = float("inf"), float("nan")
+    calls = [(lambda x, s: kernels.int4_linear(x.cuda(), packed.cuda(), s.cuda(), zero.cuda()), scale, odd4),
+             (lambda x, s: kernels.w8a16(x.cuda(), weight.cuda(), s.cuda(), False, group, 1), scale8, odd8)]
+    for call, plain, spoiled in calls:
+        want = call(x, plain).cpu()
+        got = call(odd, plain).cpu()
+        rest = [i for i in range(rows) if i not in (3, 7)]
+        assert not bool(torch.isfinite(got[[3, 7]]).any()) and bool(torch.isinf(got[3]).all())
+        assert torch.equal(got[rest], want[rest])
+        got = call(x, spoiled).cpu()
+        rest = [i for i in range(out) if i not in (11, 600)]
+        assert bool(torch.isnan(got[:, 600]).all()) and not bool(torch.isfinite(got[:, 11]).any())
+        assert torch.equal(got[:, rest], want[:, rest])
 
 
 def test_slow_scales_do_not_outrun_the_weights():
