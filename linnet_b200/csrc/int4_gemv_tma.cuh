@@ -359,7 +359,8 @@ int4_gemv_tma_kernel(const __grid_constant__ CUtensorMap wmap, const TmaArgs a) 
     int n = 0;                      // items this warp has taken
     int s = warp % S;               // stage of its next item: the items before it in the producer's order, modulo S
     const int s_step = active % S;  // a full round's items between two of this warp's
-    const int s_last = (min(a.tpc, t1 - t0 - (rounds - 1) * a.tpc) * a.wpt) % S;  // the last round's
+    const int last_round = t0 + (rounds - 1) * a.tpc;  // its first tile (a warp's own last tile may be in the round before)
+    const int s_last = (min(a.tpc, t1 - last_round) * a.wpt) % S;  // the last round's
     const uint32_t ready = ready0 + warp * 8;
     for (int tile = t0 + ts, round = 0; tile < t1; tile += a.tpc, ++round) {
         float acc[MB][2][4];
@@ -383,7 +384,7 @@ int4_gemv_tma_kernel(const __grid_constant__ CUtensorMap wmap, const TmaArgs a) 
                 if (next_tile < t1) load_sz(next_tile, more_here ? item + 1 : part * a.opc, szr);
             }
             s_mine = s;
-            s += tile + a.tpc >= t1 ? s_last : s_step;
+            s += tile >= last_round ? s_last : s_step;
             if (s >= S) s -= S;
             stage_addr = smem0 + uint32_t(s_mine) * kItem;
             if (ok) ok = bar_wait(ready, uint32_t(n) & 1, a.status, 12);

@@ -188,7 +188,8 @@ int8_gemv_tma_kernel(const __grid_constant__ CUtensorMap wmap, const Tma8Args a)
     int n = 0;
     int s = warp % S;
     const int s_step = active % S;
-    const int s_last = (min(a.tpc, t1 - t0 - (rounds - 1) * a.tpc) * a.wpt) % S;
+    const int last_round = t0 + (rounds - 1) * a.tpc;  // its first tile (a warp's own last tile may be in the round before)
+    const int s_last = (min(a.tpc, t1 - last_round) * a.wpt) % S;
     const uint32_t ready = ready0 + warp * 8;
     for (int tile = t0 + ts; tile < t1; tile += a.tpc) {
         float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
@@ -197,7 +198,7 @@ int8_gemv_tma_kernel(const __grid_constant__ CUtensorMap wmap, const Tma8Args a)
         for (int o = 0; o < a.opc; ++o, ++n) {
             const int item = part * a.opc + o;
             s_mine = s;
-            s += tile + a.tpc >= t1 ? s_last : s_step;
+            s += tile >= last_round ? s_last : s_step;
             if (s >= S) s -= S;
             stage_addr = smem0 + uint32_t(s_mine) * kItem;
             if (ok) ok = bar_wait(ready, uint32_t(n) & 1, a.status, 22);
