@@ -130,10 +130,7 @@ int4_gemv_tma_kernel(const __grid_constant__ CUtensorMap wmap, const TmaArgs a) 
     if (warp == WARPS) {
         // ---- producer: items in the order (round, item of the tile, consumer) ----------------
         if (lane != 0) return;
-        if (a.overlap) pdl_launch_dependents();
-        // Weights are constants: each consumer's first item goes out ahead of the kernel before this
-        // one.  The bounded waits come after it, since the consumers wait for the activations first.
-        bool waited = !a.overlap;
+        if (a.overlap) pdl_launch_dependents();  // this thread never waits on the previous kernel: weights are constants
         int s = 0;
         uint32_t lap = 0;  // times the ring has been gone round
         bool ok = true;
@@ -146,7 +143,6 @@ int4_gemv_tma_kernel(const __grid_constant__ CUtensorMap wmap, const TmaArgs a) 
                     const int tile = t0 + round * a.tpc + ts;
                     for (int part = 0; part < a.wpt; ++part, ++w) {
                         const uint32_t empty = empty0 + s * 8, ready = ready0 + w * 8;
-                        if (!waited && (lap > 0 || n > 0)) pdl_wait(), waited = true;
                         if (lap > 0) ok = bar_wait<true>(empty, (lap - 1) & 1, a.status, 11);
                         if (ok && n > 0) ok = bar_wait<true>(taken0 + w * 8, (n - 1) & 1, a.status, 13);
                         if (!ok) break;

@@ -116,10 +116,7 @@ int8_gemv_tma_kernel(const __grid_constant__ CUtensorMap wmap, const Tma8Args a)
         // them a consumer's in `producers` and with it a stage's ------------------------------------
         const int mine = warp - WARPS, producers = a.producers;
         if (lane != 0 || mine >= producers) return;
-        if (a.overlap) pdl_launch_dependents();
-        // Weights are constants: each consumer's first item goes out ahead of the kernel before this
-        // one.  The bounded waits come after it, since the consumers wait for the activations first.
-        bool waited = !a.overlap;
+        if (a.overlap) pdl_launch_dependents();  // this thread never waits on the previous kernel: weights are constants
         int s = mine;
         uint32_t lap = 0;  // times the ring has been gone round
         bool ok = true;
@@ -130,7 +127,6 @@ int8_gemv_tma_kernel(const __grid_constant__ CUtensorMap wmap, const Tma8Args a)
                 int tile = t0 + round * a.tpc, part = mine;
                 for (int w = mine; w < tiles_here * a.wpt; w += producers) {
                     const uint32_t empty = empty0 + s * 8, ready = ready0 + w * 8;
-                    if (!waited && (lap > 0 || n > 0)) pdl_wait(), waited = true;
                     if (lap > 0) ok = bar_wait<true>(empty, (lap - 1) & 1, a.status, 21);
                     if (ok && n > 0) ok = bar_wait<true>(taken0 + w * 8, (n - 1) & 1, a.status, 23);
                     if (!ok) break;

@@ -106,20 +106,26 @@ __device__ __forceinline__ bool bar_test_wait(uint32_t bar, uint32_t parity) {  
         : "memory");
     return ok != 0;
 }
-// Bounded wait: false (and the status word set) after about a second, or as soon as another
-// warp of the device has given up.  SPIN: poll without suspending (the producer, one thread,
+// Bounded wait: false (and the status word set) after about a second (another one when the kernels
+// before this one are done: see umma::mbar_wait), or as soon as another warp of the device has given up.  SPIN: poll without suspending (the producer, one thread,
 // which should see a freed stage at once); otherwise the hardware may park the warp a while.
 template <bool SPIN = false>
 __device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity, int* status, int code) {
     if (SPIN ? bar_test_wait(bar, parity) : bar_try_wait(bar, parity)) return true;
-    const uint64_t start = umma::global_timer_ns();
+    uint64_t start = umma::global_timer_ns();
+    bool alone = false;  // the kernels before this one are done
     for (uint32_t spins = 0;; ++spins) {
         if (SPIN ? bar_test_wait(bar, parity) : bar_try_wait(bar, parity)) return true;
         if ((spins & 1023u) == 1023u) {
             if (*reinterpret_cast<volatile int*>(status) != 0) return false;
             if (umma::global_timer_ns() - start > 1000000000ull) {
-                atomicCAS(status, 0, code);
-                return false;
+                if (alone) {
+                    atomicCAS(status, 0, code);
+                    return false;
+                }
+                pdl_wait();
+                alone = true;
+                start = umma::global_timer_ns();
             }
         }
     }

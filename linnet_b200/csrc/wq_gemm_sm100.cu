@@ -28,9 +28,6 @@
 // shared memory, in the order of the slices.  No global scratch, no atomics on results.
 // Every wait on an mbarrier is bounded: on expiry the block raises an error flag in global memory,
 // stops issuing work, waits for its copies in flight, still releases its tensor memory and returns.
-// The bounds are for work of this kernel only.  Launched early, a role waits for the kernels before
-// this one (pdl_wait, as long as they take: a reduction over ranks may wait many seconds for its
-// peers) ahead of the first of its waits that depends on the activations.
 //
 // What bounds it: the dequantizers' integer pipe for few rows (about 700 clocks an item, 28 weights a
 // clock and multiprocessor), the tensor pipe and the chip's power for prompts.  In a chain of launches
@@ -352,9 +349,7 @@ wq_gemm_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant_
         }
     } else if (warp == kWWarp) {
         if (lane == 0) {
-            // (a fetch ahead ends with the first lap: whoever frees a stage waits for the activations)
-            bool waited = a.wait_weights;
-            if (waited) pdl_wait();
+            if (a.wait_weights) pdl_wait();
             int s = 0;
             uint32_t lap = 0;
             bool ok = true;
@@ -362,10 +357,7 @@ wq_gemm_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant_
                 const int n0 = (tile / a.m_tiles) * R * kTileRows;
                 for (int c = chunk0; c < chunk1 && ok; ++c) {
                     for (int r = 0; r < R && ok; ++r) {
-                        if (lap > 0) {
-                            if (!waited) pdl_wait(), waited = true;
-                            ok = mbar_wait(&pipe->empty_w[s], (lap - 1) & 1, &g_gemm_error, 2);
-                        }
+                        if (lap > 0) ok = mbar_wait(&pipe->empty_w[s], (lap - 1) & 1, &g_gemm_error, 2);
                         if (!ok) break;
                         mbar_expect_tx(&pipe->full_w[s], kWStage);
                         tma_load_2d(smem + a.w_ring + size_t(s) * kWStage, &w_map, c * kRowBytes, n0 + r * kTileRows,
@@ -394,7 +386,6 @@ wq_gemm_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant_
         const bool leader = elect_one();
         const uint64_t x_desc = smem_desc(smem_u32(smem));
         const uint32_t half_step = x_half >> 4, stage_step = x_stage >> 4;
-        pdl_wait();
         uint32_t t = 0, item0 = 0, x0 = 0;  // tiles, items and stages of X before this tile
         bool ok = true;
         for (int tile = tile_first; tile < a.tiles && ok; tile += tile_stride, ++t) {
@@ -442,10 +433,7 @@ wq_gemm_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant_
         const uint32_t lane_base = tmem + (uint32_t(warp & 3) << 21) + a_columns + uint32_t(half) * (kStep / 2);
         const int c_step = R == 2 ? 1 : 2;
         const int ks_real = a.K / kStep;
-        // The items of the first lap of the slots need nothing of the kernels before this one; w_stages
-        // is no less than slots, so the stages of W they come from are not refilled ones either.
-        bool waited = a.wait_weights;
-        if (waited) pdl_wait();
+        if (a.wait_weights) pdl_wait();
         uint32_t item0 = 0;  // items before this tile
         bool ok = true;
         for (int tile = tile_first; tile < a.tiles && ok; tile += tile_stride) {
@@ -469,7 +457,6 @@ wq_gemm_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant_
                 const ItemScales<FORMAT, GPS> now = next;
                 next = after;
                 if (c + 2 * c_step < chunk1) after = scales_of(c + 2 * c_step);
-                if (lap > 0 && !waited) pdl_wait(), waited = true;
                 ok = warp_wait(&pipe->full_w[s], phase, 6);
                 if (!ok) break;
                 const uint32_t to = lane_base + slot * kSlotColumns;
@@ -542,7 +529,6 @@ wq_gemm_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant_
         // ---- epilogue (warp w owns tensor-memory lanes 32w .. 32w+31) ----
         float* exchange = reinterpret_cast<float*>(smem + a.exchange);
         const int cps = (nx + splits - 1) / splits;  // K slices: columns this block adds up
-        pdl_wait();
         uint32_t t = 0, item0 = 0;
         bool ok = true;
         for (int tile = tile_first; tile < a.tiles && ok; tile += tile_stride, ++t, item0 += uint32_t(span * R)) {
