@@ -29,14 +29,18 @@
 // Every wait on an mbarrier is bounded: on expiry the block raises an error flag in global memory,
 // stops issuing work, waits for its copies in flight, still releases its tensor memory and returns.
 //
-// What bounds it: the dequantizers' integer pipe for few rows (about 700 clocks an item, 28 weights a
-// clock and multiprocessor), the tensor pipe and the chip's power for prompts.  In a chain of launches
-// on a B200, us, against the kernels this one took over from (decode kernels in passes, a bf16-only
-// tensor-core kernel with dequantized weights in shared memory):
-//   int4 g128 bf16    16 x 14336 -> 4096   26.6 -> 18.4     128 x 4096 -> 28672   58 -> 34
-//                   2048 x 4096 -> 28672  392 -> 375..400 (power)
-//   int4 g32           16 x 4096 -> 28672 109.7 -> 30.5
-//   int8               64 x 4096 -> 14336 154.8 -> 20.5     200 x 4096 -> 14336  508.6 -> 29.8
+// What bounds it: for few rows no unit (ncu, 16 x 14336 -> 4096 and 100 x 4096 -> 28672: integer pipe 38 and
+// 49 % busy, issue 50 and 62 %, tensor pipe 5 and 48 %, DRAM under 20 %), but an item's way through its
+// roles and the multiprocessors left without a tile; for prompts the tensor pipe (72 % busy at
+// 2048 x 4096 -> 28672) and the chip's power.  In a chain of launches on a B200, us, against the kernels
+// this one took over from (decode kernels in passes, a bf16-only tensor-core kernel with dequantized
+// weights in shared memory):
+//   int4 g128 bf16    16 x 14336 -> 4096   25.7 -> 18.5     128 x 4096 -> 28672   47 -> 34
+//                   2048 x 4096 -> 28672  383..488 -> 362..418 (power)
+//   int4 g32           16 x 4096 -> 28672 110.4 -> 30.9
+//   int8               64 x 4096 -> 14336 155.7 -> 19.8     200 x 4096 -> 14336  501.7 -> 27.8
+// Slower than the kernel before at two sizes found: 256 x 4096 -> 28672 54 -> 58 and 512 x 4096 -> 14336
+// 53 -> 57, where its tiles of 128 columns leave half of a second round of multiprocessors idle.
 #include <atomic>
 
 #include "mma.cuh"
@@ -740,17 +744,29 @@ int resident_clusters(int splits) {
     return count;
 }
 
-// The tile shape and K split with the least estimated time: rounds of tiles times a tile's clocks.
-// An item (128 inputs x 128 rows of W) takes the products kProductClocks a column (kWideX times
-// that where one block of rows is fed from wide tiles of X: shared memory), the dequantizers
-// kItemClocks and one issuing warp kIssueClocks; a tile that cannot double-buffer its accumulators
-// pays kColumnClocks a column for its epilogue, a K split kSplitClocks and kExchangeClocks a column.
-// The constants are fitted to 1,000 measured launches (16 to 2048 rows on five weights, every tile
-// shape); the shapes they choose are within 1.6 % of the best measured ones on average.
-constexpr double kItemClocks = 766, kIssueClocks = 1031, kTileClocks = 1200, kSplitClocks = 3200, kExchangeClocks = 78,
-                 kColumnClocks = 48, kProductClocks = 3.5, kWideX = 1.58;
+// The tile shape and K split with the least estimated time: rounds of tiles times a tile's clocks, and
+// what a launch pays once.  An item (128 inputs x 128 rows of W) takes the products `product` a column
+// (`wide` times that where one block of rows is fed from wide tiles of X: shared memory), the
+// dequantizers `item` and one issuing warp `issue`.  A tile takes `tile` and `tile_column` a column, with K
+// split `split_tile` and `exchange_tile` a column more; one that cannot double-buffer its accumulators
+// `column` a column for its epilogue, which the others pay once a launch.  `split`, `exchange`: once a
+// launch with K split.
+struct PlanClocks {
+    double item, issue, product, wide, tile, tile_column, column, split_tile, exchange_tile, split, exchange;
+};
+// Fitted to the launches of every tile shape at 16 to 2048 rows on five weights.  They serve up to 64 rows,
+// and fine groups (several scales an item and row: the dequantizers take longer) at any.
+constexpr PlanClocks kFewRows = {766, 1031, 3.5, 1.58, 1200, 0, 48, 3200, 78, 0, 0};
+// Fitted to the launches of every tile shape at 100 sizes of more rows (to 2048, 2048 to 14336 inputs, 1024
+// to 28672 columns), each shape counting by how near its estimate comes to the least, so that no size
+// hangs on a rounding: the shapes chosen are 0.6 % slower than the best measured ones on average, 1.7 %
+// at the 90th percentile, 13 % at the worst (1500 x 14336 -> 2048: 87.6 us against 77.8).  2048 x 14336 -> 4096
+// takes 160 columns and two issuers, 198 us; with kFewRows it took 240 and one, 218 to 230.
+constexpr PlanClocks kManyRows = {580, 1040, 3.43, 1.2, 4000, 0, 18, 4600, 130, 0, 0};
+constexpr int64_t kManyFrom = 65;
 
-bool choose_plan(const WqProblem& q, WqPlan* best) {
+// The estimate's clocks, 0 where nothing fits.
+double choose_plan(const WqProblem& q, const PlanClocks& k, WqPlan* best) {
     const int chunks = int((q.in + kChunk - 1) / kChunk);
     double best_cost = 0;
     bool found = false;
@@ -769,18 +785,19 @@ bool choose_plan(const WqProblem& q, WqPlan* best) {
                 p.nx = nx, p.R = R, p.issuers = issuers, p.splits = splits, p.m_tiles = int(m_tiles), p.n_tiles = n_tiles;
                 if (!lay_out(p, q.format)) continue;
                 const int64_t tiles = m_tiles * n_tiles, slots = resident_clusters(splits);
-                double item = kProductClocks * nx * (R == 1 && nx > 128 ? kWideX : 1.0);
-                if (item < kItemClocks) item = kItemClocks;
-                if (issuers == 1 && item < kIssueClocks) item = kIssueClocks;
-                const double epilogue = kColumnClocks * R * nx;
-                const double tile = double((chunks + splits - 1) / splits) * R * item + (splits > 1 ? kSplitClocks + kExchangeClocks * nx : 0) +
-                                    kTileClocks + (p.acc_bufs == 1 ? epilogue : 0);
-                const double cost = double((tiles + slots - 1) / slots) * tile + (p.acc_bufs == 2 ? epilogue : 0);
+                double item = k.product * nx * (R == 1 && nx > 128 ? k.wide : 1.0);
+                if (item < k.item) item = k.item;
+                if (issuers == 1 && item < k.issue) item = k.issue;
+                const double epilogue = k.column * R * nx;
+                const double tile = double((chunks + splits - 1) / splits) * R * item + k.tile + k.tile_column * nx +
+                                    (splits > 1 ? k.split_tile + k.exchange_tile * nx : 0) + (p.acc_bufs == 1 ? epilogue : 0);
+                const double cost = double((tiles + slots - 1) / slots) * tile + (p.acc_bufs == 2 ? epilogue : 0) +
+                                    (splits > 1 ? k.split + k.exchange * nx : 0);
                 if (!found || cost < best_cost) *best = p, best_cost = cost, found = true;
             }
         }
     }
-    return found;
+    return best_cost;
 }
 
 }  // namespace
@@ -799,7 +816,8 @@ int32_t wq_gemm(const char* who, const WqProblem& q, WqStart start, cudaStream_t
     EncodeTiled encode = encode_tiled();
     if (encode == nullptr) return unavailable("%s: the driver has no cuTensorMapEncodeTiled", who);
     WqPlan p;
-    if (!choose_plan(q, &p)) return fail("%s: no tile shape for %lld rows", who, (long long)q.rows);
+    const bool fine = q.group < kStep;
+    if (choose_plan(q, q.rows < kManyFrom || fine ? kFewRows : kManyRows, &p) <= 0) return fail("%s: no tile shape for %lld rows", who, (long long)q.rows);
 
     const cuuint32_t elem[2] = {1, 1};
     CUtensorMap x_map, w_map;
