@@ -316,24 +316,22 @@ int32_t dispatch_gemv(const GemvArgs& a, const Plan& p, cudaStream_t stream) {
     return launch_gemv<T, MODE, 2, 2, 4, 2>(a, p.ksplit, stream);
 }
 
-// Three or more rows: the kernel that stages the activations once per block.  Picks the
-// warps (tiles) per block so that every block of the grid is resident at once, and the
-// octs per block so that the cluster has at most 8 blocks.
 bool rows_kernel_takes(const GemvArgs& a) {
     return a.G == 128 && a.K % 1024 == 0 && aligned(a.scale, 16) && aligned(a.zero, 8);
 }
 
-template <typename T, int MB>
-bool run_rows(const GemvArgs& a, cudaStream_t stream, int32_t* status) {
-    if (!rows_kernel_takes(a)) return false;
-    const int octs = a.K / 1024;
-    int opc = 0;
-    for (int c = 1; c <= octs; ++c)
-        if (octs % c == 0 && octs / c <= 8) { opc = c; break; }
-    if (opc == 0) return false;
-    RowsArgs r{a.x, a.packed, a.scale, a.zero, a.y, a.M, a.K, a.N, (a.N + 15) / 16, opc, octs / opc,
-               (a.flags & B200Q_NO_OVERLAP) ? 0 : 1};
-    const int sms = sm_count();
+// Three or more rows: the kernel that stages the activations once per block.  Picks the
+// warps (tiles) per block so that every block of the grid is resident at once, and the
+// octs per block so that the cluster has at most 8 blocks.
+struct RowsGrid {
+    int warps, octs_per_block, ksplit, blocks;
+};
+template <int MB>
+RowsGrid rows_grid(const GemvArgs& a) {
+    const int octs = a.K / 1024, tiles = (a.N + 15) / 16;
+    int opc = 1;
+    while (octs % opc != 0 || octs / opc > 8) ++opc;
+    const int ksplit = octs / opc, sms = sm_count();
     // Widest block (most sharing of the staged activations) among those that keep every
     // block resident at once and still put a block on every multiprocessor.
     const int candidates[4] = {14, 7, 4, 2};
@@ -348,13 +346,22 @@ bool run_rows(const GemvArgs& a, cudaStream_t stream, int32_t* status) {
         const int by_regs = w == 14 && warps_by_regs < 14 ? 1 : warps_by_regs / w;
         if (by_smem < 1 || by_regs < 1) continue;
         const int resident = sms * (by_smem < by_regs ? by_smem : by_regs);
-        const int blocks = ((r.tiles + w - 1) / w) * r.ksplit;
+        const int blocks = ((tiles + w - 1) / w) * ksplit;
         const double waves = double((blocks + resident - 1) / resident);
         const double coverage = blocks >= sms ? 1.0 : double(blocks) / double(sms);
         const double cost = waves / coverage;
         if (cost < best_cost - 1e-9) { best_cost = cost; best = w; }
     }
-    switch (best) {
+    return {best, opc, ksplit, ((tiles + best - 1) / best) * ksplit};
+}
+
+template <typename T, int MB>
+bool run_rows(const GemvArgs& a, cudaStream_t stream, int32_t* status) {
+    if (!rows_kernel_takes(a)) return false;
+    const RowsGrid g = rows_grid<MB>(a);
+    RowsArgs r{a.x, a.packed, a.scale, a.zero, a.y, a.M, a.K, a.N, (a.N + 15) / 16, g.octs_per_block, g.ksplit,
+               (a.flags & B200Q_NO_OVERLAP) ? 0 : 1};
+    switch (g.warps) {
         case 4: *status = launch_rows<T, MB, 4, 2>(r, stream); break;
         case 7: *status = launch_rows<T, MB, 7, 2>(r, stream); break;
         case 14: *status = launch_rows<T, MB, 14, 2>(r, stream); break;
@@ -517,6 +524,19 @@ int32_t run_gemv(GemvArgs a, int64_t rows, cudaStream_t stream) {
 }
 
 }  // namespace
+
+double rows_kernel_us(const WqProblem& p) {
+    const GemvArgs a{p.x, static_cast<const uint8_t*>(p.weight), p.scale, p.zero, p.y, 16, int(p.in), int(p.out),
+                     int(p.group), int(p.in / 128), 0, 1, 0};
+    if (!rows_kernel_takes(a)) return -1.0;
+    const RowsGrid g = rows_grid<2>(a);
+    // Blocks a multiprocessor takes in all, a twentieth more than their number says: clusters do not
+    // fill every multiprocessor.  Two 14-warp blocks run side by side.
+    const int each = int((g.blocks * 21 / 20 + sm_count() - 1) / sm_count());
+    if (g.warps != 14 || each > 4) return 1e9;
+    constexpr double kOneOct[4] = {10.9, 15.0, 24.0, 30.2}, kNextOct = 10.9;
+    return kOneOct[each - 1] + (g.octs_per_block - 1) * kNextOct;
+}
 
 int64_t int4_unrounded_rows(const WqProblem& p, int32_t flags) {
     if (flags & B200Q_EXACT_WEIGHTS) return 0;

@@ -297,11 +297,11 @@ constexpr int64_t kOverlapRows8 = 64;
 // stay with the decode kernels: those with one scale a row with int8_gemv_tma.cuh's, whose sums take
 // the scale unrounded, those with group scales came out 0.86 to 1.25 times over drawn shapes).
 // Decode kernel / tensor-core product, us a launch in a chain on a B200:
-//                                 1 row     3 rows     6 rows     8 rows    16 rows
-//   2048 -> 2048                5.2/7.9    5.6/7.9    5.9/8.0    6.0/8.0    8.3/8.0
-//   4096 -> 4096               9.4/10.5   9.9/10.7  10.4/11.0  15.7/11.0  12.3/11.0
-//   4096 -> 14336             22.0/18.0  23.7/17.9  31.4/17.9  32.5/17.9  40.7/18.0
-//   14336 -> 4096             24.8/19.5  34.2/19.9  35.5/20.2  36.9/20.2  45.2/20.2
+//                                           3 rows     6 rows     8 rows    16 rows
+//   2048 -> 2048                           5.6/7.7    5.8/7.7    6.0/7.7    8.4/7.8
+//   4096 -> 4096                         10.1/11.2  10.6/11.4  15.9/11.4  12.7/11.5
+//   4096 -> 14336                        24.4/18.9  31.8/18.9  33.1/18.9  41.2/18.9
+//   14336 -> 4096                        34.0/21.1  35.8/21.3  37.3/21.2  45.7/21.3
 int64_t gemm_rows8(int64_t weights) {
     if (weights < (int64_t(6) << 20)) return 14;   // 1536 x 4096 (2048 x 1536, 13 rows: 6.5/7.2)
     if (weights < (int64_t(12) << 20)) return 9;   // 3072 x 4096

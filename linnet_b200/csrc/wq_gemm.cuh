@@ -32,6 +32,13 @@ enum class WqStart {
 };
 int32_t wq_gemm(const char* who, const WqProblem& p, WqStart start, cudaStream_t stream);
 
+// The time a launch for up to 16 rows is expected to take, by the estimate its tile shape is chosen with.
+double wq_gemm_us(const WqProblem& p);
+
+// int4_gemv.cu: the same of the decode kernel that 9 to 16 rows of groups of 128 get; -1 where that is
+// another one than the kernel with shared activations.
+double rows_kernel_us(const WqProblem& p);
+
 // int4_gemv.cu: of this many rows, how many at the end the decode kernels' passes of 16 (or 64) leave
 // to the one- and two-row kernel, whose sums take zero point and scale unrounded.
 int64_t int4_unrounded_rows(const WqProblem& p, int32_t flags);

@@ -764,6 +764,8 @@ constexpr PlanClocks kFewRows = {766, 1031, 3.5, 1.58, 1200, 0, 48, 3200, 78, 0,
 // takes 160 columns and two issuers, 198 us; with kFewRows it took 240 and one, 218 to 230.
 constexpr PlanClocks kManyRows = {580, 1040, 3.43, 1.2, 4000, 0, 18, 4600, 130, 0, 0};
 constexpr int64_t kManyFrom = 65;
+// Fitted to the times themselves at 16 to 64 rows: for the choice between this kernel and another.
+constexpr PlanClocks kFewRowsTime = {470, 620, 3.2, 1.2, 520, 54, 144, 0, 0, 4870, 95};
 
 // The estimate's clocks, 0 where nothing fits.
 double choose_plan(const WqProblem& q, const PlanClocks& k, WqPlan* best) {
@@ -801,6 +803,12 @@ double choose_plan(const WqProblem& q, const PlanClocks& k, WqPlan* best) {
 }
 
 }  // namespace
+
+double wq_gemm_us(const WqProblem& q) {
+    WqPlan p;
+    const double clocks = choose_plan(q, kFewRowsTime, &p);
+    return clocks > 0 ? clocks / 1155 - 1.06 : 1e9;  // 300 launches of 9 to 16 rows: 4 % off in the middle, 20 at the 90th percentile
+}
 
 bool wq_gemm_supports(const WqProblem& p) {
     const bool fine = p.group == 16 || p.group == 32 || (p.group > 0 && p.group % kStep == 0);

@@ -177,6 +177,22 @@ def test_unaligned_activations_keep_the_library_route():
     check(got, x[1:].view(100, 512), lo.int8_weight(weight, scale.reshape(-1), torch.bfloat16))
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize(("rows", "depth", "out"), [
+    (9, 8192, 5120), (16, 8192, 7168), (12, 4096, 14336), (16, 12288, 4608),  # the decode kernel's
+    (9, 4096, 16384), (16, 8192, 8192), (12, 2048, 5120), (16, 1024, 1024), (11, 7168, 2050), (17, 8192, 5120),  # the product's
+])
+def test_int4_nine_to_sixteen_rows(rows, depth, out, dtype):
+    """Either kernel may take these rows of groups of 128, by its estimated time; both round every
+    weight once."""
+    from linnet_b200 import kernels
+
+    gen = torch.Generator().manual_seed(rows + depth + out)
+    packed, scale, zero = make_int4(out, depth, 128, dtype, gen, 0.02)
+    x = torch.randn(rows, depth, generator=gen).to(dtype)
+    check(kernels.int4_linear(x.cuda(), packed.cuda(), scale.cuda(), zero.cuda()), x, lo.int4_weight(packed, scale, zero, dtype))
+
+
 @pytest.mark.parametrize(("rows", "depth", "out", "dtype"), [
     (17, 1536, 4096, torch.bfloat16), (18, 5632, 1000, torch.bfloat16), (33, 1536, 4096, torch.float16),
     (50, 2560, 4096, torch.float16), (65, 2048, 4096, torch.float16), (130, 4096, 4096, torch.float16),
