@@ -79,7 +79,7 @@ int32_t b200q_int4_linear(const void* x, const uint8_t* packed, const void* scal
                           const uint8_t* zero, void* y, int64_t rows, int64_t in,
                           int64_t out, int64_t group, int32_t dtype, void* stream);
 
-/* The decode kernel alone: rows <= 16, HBM-bound weight streaming. */
+/* The decode kernels alone: a few rows, weight streaming (more rows run in passes). */
 int32_t b200q_int4_gemv(const void* x, const uint8_t* packed, const void* scale,
                         const uint8_t* zero, void* y, int64_t rows, int64_t in,
                         int64_t out, int64_t group, int32_t dtype, void* stream);
@@ -148,8 +148,8 @@ int32_t b200q_int4_gemv_norm(const void* x, const void* delta, const void* norm_
                              int64_t group, int32_t dtype, int32_t flags, void* stream);
 
 /* Synchronises the device and reports whether any launch on it of a kernel with a
- * shared-memory pipeline (b200q_int4_gemm, b200q_int8_mm, the one- and two-row kernel of
- * b200q_int4_gemv / b200q_int4_linear) gave up on one of its bounded waits (B200Q_ERROR,
+ * shared-memory pipeline (the tensor-core products of int4 and int8 weights, b200q_int8_mm, the one- and
+ * two-row kernels) gave up on one of its bounded waits (B200Q_ERROR,
  * with the waiting role in the message); such a launch leaves its output incomplete but the context usable.  Reporting clears
  * the condition (until then later launches cut their waits short).  No reference
  * counterpart: the reference's kernels spin without a bound. */

@@ -426,8 +426,9 @@ int32_t launch_attention(const char* who, const void* q, const void* cache_k, co
     else if (longest_first) B200Q_ATTN_W(HD, REP, 4, true); else B200Q_ATTN_W(HD, REP, 4, false); } while (0)
     cudaError_t err = cudaSuccess;
     const bool few_blocks = splits * nkv * batch <= sm_count();
-    // two blocks of 4 warps fit on a multiprocessor, and a block ranks one row a thread
-    // 64 rows of 1024 to 2048 keys x 8 KV heads: 91.1 -> 80.3 us; all of 2048 keys: 99.4 -> 100.0
+    // Two blocks of 4 warps fit on a multiprocessor, and a block ranks one row a thread.  x 8 KV heads:
+    // 64 rows of 1024 to 2048 keys 91.1 -> 80.3 us, 48 rows 71.9 -> 72.3 (no gain); 64 rows all of
+    // 2048 keys 99.4 -> 100.0.
     const bool longest_first = splits * nkv * batch > 2 * sm_count() && batch <= 128 && max_seq < (int64_t(1) << 23);
     if (head_dim == 128) {
         if (rep == 1) B200Q_ATTN(128, 1); else if (rep == 2) B200Q_ATTN(128, 2);

@@ -14,8 +14,10 @@
 // TMA producer, one thread of warp 5 issues the MMAs (128 x BN x 32 per instruction, four per
 // 128-byte stage), warps 0-3 are the epilogue (tcgen05.ld -> f32 -> scales -> 16-bit -> y).
 // One persistent block per multiprocessor walks over the 128 x BN tiles; the accumulators are
-// double-buffered so a tile's epilogue overlaps the next tile's products.  Every mbarrier
-// wait is bounded (shared with the int4 GEMM: b200q_int4_gemm_status() reports an expiry).
+// double-buffered so a tile's epilogue overlaps the next tile's products.  More than 128 rows mostly
+// run the form for pairs of multiprocessors (int8_mm_pair_kernel, tiles of 256 rows), which halves
+// what each reads of the weights.  Every mbarrier wait is bounded, by the status word of the
+// dequantizing product (wq_gemm_sm100.cu): b200q_int4_gemm_status() reports an expiry.
 #include <atomic>
 
 #include "mma.cuh"

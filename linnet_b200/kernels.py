@@ -159,8 +159,8 @@ def int4_linear(x: torch.Tensor, packed: torch.Tensor, scale: torch.Tensor,
                 swiglu: bool = False, overlap: bool = True) -> torch.Tensor:
     """`F.linear(x, W)` for `x` [rows, In] (bf16 or f16) and the group-wise 4-bit weight
     of `std.quant::linear_int4_groups`: `packed` [Out, Groups, Group/2] u8 (even value
-    low), `scale` and `zero` [Out, Groups].  Any row count: up to 16 rows stream the
-    weight once at HBM speed, more go through the tensor-memory GEMM.  `out` (eager
+    low), `scale` and `zero` [Out, Groups].  Any row count: a few rows stream the weight once
+    through the decode kernels, more through the tensor-core product.  `out` (eager
     calls only) receives the result in place of a new tensor, e.g. a buffer in peer-mapped
     memory that a tensor-parallel reduction reads next.  `early` (eager calls only): the next
     kernel in the stream is another product of the same input, which may start prefetching its

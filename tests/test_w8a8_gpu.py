@@ -36,8 +36,8 @@ def test_int8_rows_is_exact(rows, depth, dtype):
 @pytest.mark.parametrize(("rows", "depth", "out"), [
     (33, 128, 16), (64, 512, 72), (128, 4096, 4096), (129, 1024, 272), (300, 4096, 1000), (2048, 4096, 6144),
     (2048, 14336, 4096), (1, 256, 48),
-    # wide tiles whose width is chosen by how the tiles fill the multiprocessors (224, 240 rows of W
-    # on 148 of them), ragged last tiles, an output width that is no multiple of 8
+    # prompts over wide weights (the tile's width is chosen by how the tiles fill the
+    # multiprocessors), ragged last tiles, an output width that is no multiple of 8
     (2048, 256, 14336), (1200, 128, 5001), (1500, 128, 9000),
 ])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
@@ -61,9 +61,9 @@ def test_int8_mm_is_exact(rows, depth, out, dtype):
 @pytest.mark.parametrize("rows", [1, 3, 17, 64, 65, 128, 300, 2048])
 @pytest.mark.parametrize("rounded", [0, 1])
 def test_int8_linear_rows_and_routes(rows, rounded):
-    """Every row-count route of `int8_linear`: the decode kernel (1, 2..64 rows), the
-    dequantized weight and the library GEMM (more rows, weight-only), int8 activations (more
-    than 32 rows with `rounded`)."""
+    """Every row-count route of `int8_linear`: the decode kernels, the tensor-core product on 16-bit
+    activations (a few rows to many, weight-only), int8 activations (more than 32 rows with
+    `rounded`)."""
     from linnet_b200 import quantized
 
     depth, out = 4096, 1024
