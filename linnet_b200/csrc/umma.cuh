@@ -51,17 +51,17 @@ __device__ __forceinline__ uint32_t clock_ticks() { return uint32_t(global_timer
 // kernels before it, which take as long as they take (a reduction over ranks may wait many seconds
 // for its peers): when the second is over those are waited for, and the wait has another second.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* error, int code) {
-#pragma unroll 1
-    for (int i = 0; i < 32; ++i)
-        if (mbar_try_wait(bar, parity)) return true;
-    uint32_t start = clock_ticks();  // its low bit: the kernels before this one are done
+    uint32_t start = 0;  // not looked at yet; its low bit: the kernels before this one are done
 #pragma unroll 1
     for (;;) {
 #pragma unroll 1
         for (int i = 0; i < 32; ++i)
             if (mbar_try_wait(bar, parity)) return true;
         if (*reinterpret_cast<volatile int*>(error) != 0) return false;  // someone else gave up
-        if (clock_ticks() - (start & ~1u) > 16) {
+        const uint32_t now = clock_ticks();
+        if (start == 0) {
+            start = now;
+        } else if (now - (start & ~1u) > 16) {
             if (start & 1u) {
                 atomicCAS(error, 0, code);
                 return false;
