@@ -23,6 +23,7 @@
 //   * the warps of a block split K; a cluster of blocks may split it further, the
 //     partial sums meeting in (distributed) shared memory, so no global scratch
 //     and no atomics are used.
+#include <atomic>
 #include <cstdlib>
 
 #include "gemv_common.cuh"
@@ -525,17 +526,50 @@ int32_t run_gemv(GemvArgs a, int64_t rows, cudaStream_t stream) {
 
 }  // namespace
 
+// 14-warp blocks of the kernel for up to 16 rows that the device holds at a time in clusters of `ksplit`;
+// asked for once per device.
+static int resident_rows_blocks(int ksplit) {
+    static std::atomic<int> cached[64][9];
+    int device = 0;
+    if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) return 2 * sm_count();
+    int count = cached[device][ksplit].load(std::memory_order_relaxed);
+    if (count == 0) {
+        const auto kernel = int4_gemv_rows_kernel<__nv_bfloat16, 2, 14, 2>;
+        ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), rows_smem(2, 14));
+        cudaLaunchConfig_t config = {};
+        config.gridDim = dim3(1, unsigned(ksplit), 1);
+        config.blockDim = dim3(14 * 32, 1, 1);
+        config.dynamicSmemBytes = rows_smem(2, 14);
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = attr[0].val.clusterDim.z = 1;
+        attr[0].val.clusterDim.y = unsigned(ksplit);
+        config.attrs = attr;
+        config.numAttrs = 1;
+        if (cudaOccupancyMaxActiveClusters(&count, kernel, &config) == cudaSuccess && count > 0) {
+            count *= ksplit;
+        } else {
+            cudaGetLastError();
+            count = 2 * sm_count();
+        }
+        cached[device][ksplit].store(count, std::memory_order_relaxed);
+    }
+    return count;
+}
+
 double rows_kernel_us(const WqProblem& p) {
     const GemvArgs a{p.x, static_cast<const uint8_t*>(p.weight), p.scale, p.zero, p.y, 16, int(p.in), int(p.out),
                      int(p.group), int(p.in / 128), 0, 1, 0};
     if (!rows_kernel_takes(a)) return -1.0;
     const RowsGrid g = rows_grid<2>(a);
-    // Blocks a multiprocessor takes in all, a twentieth more than their number says: clusters do not
-    // fill every multiprocessor.  Two 14-warp blocks run side by side.
-    const int each = int((g.blocks * 21 / 20 + sm_count() - 1) / sm_count());
-    if (g.warps != 14 || each > 4) return 1e9;
+    if (g.warps != 14) return 1e9;
+    // Two 14-warp blocks run side by side on a multiprocessor, as far as their clusters fit: 296 blocks at a
+    // time in clusters of two, 259 in clusters of seven, and one block more is another turn (8192 -> 7280,
+    // 264 blocks in clusters of eight, 16.1 us, -> 7424, 272, 22.4; 6144 -> 10000, 270 in clusters of six,
+    // 15.7, -> 10112, 276, 22.7).  The times are of 9 to 16 rows, by halves of a full house.
+    const int each = (2 * g.blocks + resident_rows_blocks(g.ksplit) - 1) / resident_rows_blocks(g.ksplit);
     constexpr double kOneOct[4] = {10.9, 15.0, 24.0, 30.2}, kNextOct = 10.9;
-    return kOneOct[each - 1] + (g.octs_per_block - 1) * kNextOct;
+    return each > 4 ? 1e9 : kOneOct[each - 1] + (g.octs_per_block - 1) * kNextOct;
 }
 
 int64_t int4_unrounded_rows(const WqProblem& p, int32_t flags) {

@@ -219,11 +219,14 @@ int4_gemv_rows_kernel(const RowsArgs a) {
     (void)owns;
 }
 
+// Shared memory of a block: staged activations of an oct, the warps' sums.
+inline size_t rows_smem(int MB, int W) { return size_t(8) * 4 * (MB * 8) * 4 * 16 + size_t(W) * 16 * (MB * 8) * 4; }
+
 // Launch geometry for the rows kernel: W warps (tiles) per block, OPC octs per block so
 // that the cluster has at most 8 blocks; false when the shape does not fit.
 template <typename T, int MB, int W, int D>
 int32_t launch_rows(RowsArgs a, cudaStream_t stream) {
-    const size_t smem = size_t(8) * 4 * (MB * 8) * 4 * 16 + size_t(W) * 16 * (MB * 8) * 4;
+    const size_t smem = rows_smem(MB, W);
     const int blocks = (a.tiles + W - 1) / W;
     return launch_clustered("int4_gemv", int4_gemv_rows_kernel<T, MB, W, D>, a, blocks, a.ksplit, W * 32,
                             smem, stream, a.overlap != 0);

@@ -29,7 +29,8 @@ static constexpr int64_t kOverlapRows = 64;
 // 9 to 16 rows with groups of 128 and inputs a multiple of 1024 go by the estimates of both kernels: the
 // decode kernel wins where its 14-warp blocks all run at once and the product has no even share for
 // the multiprocessors (9 rows 8192 -> 7168: 15.5/20.2, 4096 -> 20000: 23.5/27.6, 4096 -> 14336:
-// 15.3/15.9), the product nearly everywhere else.  For other inputs a third was lost where the
+// 15.3/15.9), the product nearly everywhere else (left: 4096 -> 5120, 10.8/12.1, 2048 -> 8192, 8.4/11.0, where
+// decode blocks of 7 warps come out just even).  For other inputs a third was lost where the
 // product's tiles of 128 columns leave its last round mostly empty and K is not split.
 static bool product_takes(const WqProblem& p) {
     constexpr int64_t kSome = int64_t(12) << 20, kMany = int64_t(32) << 20;  // weights: 3072 x 4096, 8192 x 4096
