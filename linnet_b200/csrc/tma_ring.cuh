@@ -106,8 +106,8 @@ __device__ __forceinline__ bool bar_test_wait(uint32_t bar, uint32_t parity) {  
         : "memory");
     return ok != 0;
 }
-// Bounded wait: false (and the status word set) after about a second (another one when the kernels
-// before this one are done: see umma::mbar_wait), or as soon as another warp of the device has given up.  SPIN: poll without suspending (the producer, one thread,
+// Bounded wait: false (and the status word set) after about a second, and another one when the kernels
+// before this one are done (see umma::mbar_wait), or as soon as another warp of the device has given up.  SPIN: poll without suspending (the producer, one thread,
 // which should see a freed stage at once); otherwise the hardware may park the warp a while.
 template <bool SPIN = false>
 __device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity, int* status, int code) {

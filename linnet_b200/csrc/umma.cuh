@@ -44,30 +44,25 @@ __device__ __forceinline__ uint64_t global_timer_ns() {
     asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
     return t;
 }
-// Two a 2^27 ns (0.13 s), an even number: one register for a wait's start and a bit to spare.
-__device__ __forceinline__ uint32_t clock_ticks() { return uint32_t(global_timer_ns() >> 27) << 1; }
 // Bounded wait: false (and the error flag set) after about a second.  The clock is not asked for
 // before a wait has lasted a while.  In a kernel launched early, what is waited for may hang on the
 // kernels before it, which take as long as they take (a reduction over ranks may wait many seconds
-// for its peers): when the second is over those are waited for, and the wait has another second.
+// for its peers): a wait that lasts waits for those first, and the second is for this kernel's work.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* error, int code) {
-    uint32_t start = 0;  // not looked at yet; its low bit: the kernels before this one are done
+#pragma unroll 1
+    for (int i = 0; i < 32; ++i)
+        if (mbar_try_wait(bar, parity)) return true;
+    pdl_wait();
+    const uint64_t start = global_timer_ns();
 #pragma unroll 1
     for (;;) {
 #pragma unroll 1
         for (int i = 0; i < 32; ++i)
             if (mbar_try_wait(bar, parity)) return true;
         if (*reinterpret_cast<volatile int*>(error) != 0) return false;  // someone else gave up
-        const uint32_t now = clock_ticks();
-        if (start == 0) {
-            start = now;
-        } else if (now - (start & ~1u) > 16) {
-            if (start & 1u) {
-                atomicCAS(error, 0, code);
-                return false;
-            }
-            pdl_wait();
-            start = clock_ticks() | 1u;
+        if (global_timer_ns() - start > 1000000000ull) {
+            atomicCAS(error, 0, code);
+            return false;
         }
     }
 }
