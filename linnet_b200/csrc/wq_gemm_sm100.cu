@@ -755,7 +755,9 @@ struct PlanClocks {
     double item, issue, product, wide, tile, tile_column, column, split_tile, exchange_tile, split, exchange;
 };
 // Fitted to the launches of every tile shape at 16 to 2048 rows on five weights.  They serve up to 64 rows,
-// and fine groups (several scales an item and row: the dequantizers take longer) at any.
+// and at any row count fine groups (several scales an item and row: the dequantizers take longer) and
+// odd widths (Y is stored by single columns, and the epilogue is long: 338 x 2944 -> 27815 61.5 us, with
+// kManyRows 71.9).
 constexpr PlanClocks kFewRows = {766, 1031, 3.5, 1.58, 1200, 0, 48, 3200, 78, 0, 0};
 // Fitted to the launches of every tile shape at 100 sizes of more rows (to 2048, 2048 to 14336 inputs, 1024
 // to 28672 columns), each shape counting by how near its estimate comes to the least, so that no size
@@ -824,8 +826,8 @@ int32_t wq_gemm(const char* who, const WqProblem& q, WqStart start, cudaStream_t
     EncodeTiled encode = encode_tiled();
     if (encode == nullptr) return unavailable("%s: the driver has no cuTensorMapEncodeTiled", who);
     WqPlan p;
-    const bool fine = q.group < kStep;
-    if (choose_plan(q, q.rows < kManyFrom || fine ? kFewRows : kManyRows, &p) <= 0) return fail("%s: no tile shape for %lld rows", who, (long long)q.rows);
+    const bool fine = q.group < kStep, pairs = q.out % 2 == 0 && aligned(q.y, 4);
+    if (choose_plan(q, q.rows < kManyFrom || fine || !pairs ? kFewRows : kManyRows, &p) <= 0) return fail("%s: no tile shape for %lld rows", who, (long long)q.rows);
 
     const cuuint32_t elem[2] = {1, 1};
     CUtensorMap x_map, w_map;
@@ -856,7 +858,7 @@ int32_t wq_gemm(const char* who, const WqProblem& q, WqStart start, cudaStream_t
     a.chunks = int((q.in + kChunk - 1) / kChunk);
     a.x_stages = p.x_stages, a.w_stages = p.w_stages, a.slots = p.slots, a.acc_bufs = p.acc_bufs;
     a.w_ring = uint32_t(p.w_ring), a.exchange = uint32_t(p.exchange), a.barriers = uint32_t(p.barriers);
-    a.pairs = q.out % 2 == 0 && aligned(q.y, 4);
+    a.pairs = pairs;
     a.wait_weights = start != WqStart::kFetchAhead;
 
     const WqKernel kernel = q.dtype == B200Q_BF16 ? pick<__nv_bfloat16>(q.format, q.group) : pick<__half>(q.format, q.group);
