@@ -754,22 +754,36 @@ int resident_clusters(int splits) {
 struct PlanClocks {
     double item, issue, product, wide, tile, tile_column, column, split_tile, exchange_tile, split, exchange;
 };
-// Fitted to the launches of every tile shape at 16 to 2048 rows on five weights.  They serve up to 64 rows,
-// and at any row count fine groups (several scales an item and row: the dequantizers take longer) and
-// odd widths (Y is stored by single columns, and the epilogue is long: 338 x 2944 -> 27815 61.5 us, with
-// kManyRows 71.9).
+// Fitted to the launches of every tile shape at 16 to 2048 rows on five weights.  They serve all but long
+// prompts over deep weights; those too with fine groups (several scales an item and row: the dequantizers
+// take longer) and odd widths (Y is stored by single columns, and the epilogue is long).
 constexpr PlanClocks kFewRows = {766, 1031, 3.5, 1.58, 1200, 0, 48, 3200, 78, 0, 0};
 // Fitted to the launches of every tile shape at 100 sizes of more rows (to 2048, 2048 to 14336 inputs, 1024
-// to 28672 columns), each shape counting by how near its estimate comes to the least, so that no size
-// hangs on a rounding: the shapes chosen are 0.6 % slower than the best measured ones on average, 1.7 %
-// at the 90th percentile, 13 % at the worst (1500 x 14336 -> 2048: 87.6 us against 77.8).  2048 x 14336 -> 4096
-// takes 160 columns and two issuers, 198 us; with kFewRows it took 240 and one, 218 to 230.
+// to 28672 columns), each shape counting by how near its estimate comes to the least.  Long prompts over
+// deep weights take this choice where it is the better one by both estimates together: of 38 drawn or
+// listed sizes where the two choices differ, 31 do, 4.6 % faster on average (17 % to 5 % slower; the
+// other seven came out 8 % faster to 17 % slower).  2048 x 14336 -> 4096 takes 160 columns and two issuers,
+// 196 us; kFewRows alone 240 and one, 208 to 230.  Shorter or shallower, 70 sizes came out either way.
 constexpr PlanClocks kManyRows = {580, 1040, 3.43, 1.2, 4000, 0, 18, 4600, 130, 0, 0};
-constexpr int64_t kManyFrom = 65;
+constexpr int64_t kManyFrom = 512, kDeepFrom = 3072;
+constexpr double kBoth = 0.98;
 // Fitted to the times themselves at 16 to 64 rows: for the choice between this kernel and another.
 constexpr PlanClocks kFewRowsTime = {470, 620, 3.2, 1.2, 520, 54, 144, 0, 0, 4870, 95};
 
-// The estimate's clocks, 0 where nothing fits.
+double plan_clocks(const WqProblem& q, const WqPlan& p, const PlanClocks& k) {
+    const int chunks = int((q.in + kChunk - 1) / kChunk);
+    const int64_t tiles = int64_t(p.m_tiles) * p.n_tiles, slots = resident_clusters(p.splits);
+    double item = k.product * p.nx * (p.R == 1 && p.nx > 128 ? k.wide : 1.0);
+    if (item < k.item) item = k.item;
+    if (p.issuers == 1 && item < k.issue) item = k.issue;
+    const double epilogue = k.column * p.R * p.nx;
+    const double tile = double((chunks + p.splits - 1) / p.splits) * p.R * item + k.tile + k.tile_column * p.nx +
+                        (p.splits > 1 ? k.split_tile + k.exchange_tile * p.nx : 0) + (p.acc_bufs == 1 ? epilogue : 0);
+    return double((tiles + slots - 1) / slots) * tile + (p.acc_bufs == 2 ? epilogue : 0) +
+           (p.splits > 1 ? k.split + k.exchange * p.nx : 0);
+}
+
+// The shape with the least estimate, and its clocks; 0 where nothing fits.
 double choose_plan(const WqProblem& q, const PlanClocks& k, WqPlan* best) {
     const int chunks = int((q.in + kChunk - 1) / kChunk);
     double best_cost = 0;
@@ -782,21 +796,14 @@ double choose_plan(const WqProblem& q, const PlanClocks& k, WqPlan* best) {
         tried = m_tiles;
         for (int shape = 0; shape < 3; ++shape) {
             const int R = shape == 2 ? 2 : 1, issuers = shape == 0 ? 1 : 2;
+            if (R == 1 && issuers == 2 && nx > 176) continue;  // no better than one issuer with two accumulators
             const int n_tiles = int((q.out + R * kTileRows - 1) / (R * kTileRows));
             for (int splits = 1; splits <= kMaxSplits; ++splits) {
                 if (splits > 1 && (R > 1 || nx > 128 || chunks < 2 * splits)) break;
                 WqPlan p = {};
                 p.nx = nx, p.R = R, p.issuers = issuers, p.splits = splits, p.m_tiles = int(m_tiles), p.n_tiles = n_tiles;
                 if (!lay_out(p, q.format)) continue;
-                const int64_t tiles = m_tiles * n_tiles, slots = resident_clusters(splits);
-                double item = k.product * nx * (R == 1 && nx > 128 ? k.wide : 1.0);
-                if (item < k.item) item = k.item;
-                if (issuers == 1 && item < k.issue) item = k.issue;
-                const double epilogue = k.column * R * nx;
-                const double tile = double((chunks + splits - 1) / splits) * R * item + k.tile + k.tile_column * nx +
-                                    (splits > 1 ? k.split_tile + k.exchange_tile * nx : 0) + (p.acc_bufs == 1 ? epilogue : 0);
-                const double cost = double((tiles + slots - 1) / slots) * tile + (p.acc_bufs == 2 ? epilogue : 0) +
-                                    (splits > 1 ? k.split + k.exchange * nx : 0);
+                const double cost = plan_clocks(q, p, k);
                 if (!found || cost < best_cost) *best = p, best_cost = cost, found = true;
             }
         }
@@ -826,8 +833,15 @@ int32_t wq_gemm(const char* who, const WqProblem& q, WqStart start, cudaStream_t
     EncodeTiled encode = encode_tiled();
     if (encode == nullptr) return unavailable("%s: the driver has no cuTensorMapEncodeTiled", who);
     WqPlan p;
-    const bool fine = q.group < kStep, pairs = q.out % 2 == 0 && aligned(q.y, 4);
-    if (choose_plan(q, q.rows < kManyFrom || fine || !pairs ? kFewRows : kManyRows, &p) <= 0) return fail("%s: no tile shape for %lld rows", who, (long long)q.rows);
+    if (choose_plan(q, kFewRows, &p) <= 0) return fail("%s: no tile shape for %lld rows", who, (long long)q.rows);
+    const bool pairs = q.out % 2 == 0 && aligned(q.y, 4);
+    if (q.rows >= kManyFrom && q.in >= kDeepFrom && q.group >= kStep && pairs) {
+        WqPlan other;
+        choose_plan(q, kManyRows, &other);
+        if (plan_clocks(q, other, kManyRows) * plan_clocks(q, other, kFewRows) <
+            kBoth * plan_clocks(q, p, kManyRows) * plan_clocks(q, p, kFewRows))
+            p = other;
+    }
 
     const cuuint32_t elem[2] = {1, 1};
     CUtensorMap x_map, w_map;
