@@ -112,20 +112,18 @@ __device__ __forceinline__ bool bar_test_wait(uint32_t bar, uint32_t parity) {  
 template <bool SPIN = false>
 __device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity, int* status, int code) {
     if (SPIN ? bar_test_wait(bar, parity) : bar_try_wait(bar, parity)) return true;
-    uint64_t start = umma::global_timer_ns();
-    bool alone = false;  // the kernels before this one are done
+    uint64_t start = umma::global_timer_ns() & ~uint64_t(1);  // its low bit: the kernels before this one are done
     for (uint32_t spins = 0;; ++spins) {
         if (SPIN ? bar_test_wait(bar, parity) : bar_try_wait(bar, parity)) return true;
         if ((spins & 1023u) == 1023u) {
             if (*reinterpret_cast<volatile int*>(status) != 0) return false;
             if (umma::global_timer_ns() - start > 1000000000ull) {
-                if (alone) {
+                if (start & 1) {
                     atomicCAS(status, 0, code);
                     return false;
                 }
                 pdl_wait();
-                alone = true;
-                start = umma::global_timer_ns();
+                start = umma::global_timer_ns() | 1;
             }
         }
     }
